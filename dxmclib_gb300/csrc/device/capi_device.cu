@@ -38,8 +38,8 @@ constexpr int DEFAULT_QUEUE_INTERACT_THRESHOLD = 8;
 constexpr int DEFAULT_WOODCOCK_BURST = DXMC_DEFAULT_WOODCOCK_BURST; // Woodcock steps per loop iteration
 // With local majorants a history takes fewer, more varied steps: shorter bursts
 // and a later refill keep more lanes of a warp stepping together.
-constexpr int DEFAULT_LOCAL_REGEN_THRESHOLD = 10;
-constexpr int DEFAULT_LOCAL_WOODCOCK_BURST = 4;
+constexpr int DEFAULT_LOCAL_REGEN_THRESHOLD = 4;
+constexpr int DEFAULT_LOCAL_WOODCOCK_BURST = 3;
 // Local-majorant grid: target cell edge and energy bands (above 15 keV)
 #ifndef DXMC_MAJORANT_CELL_MM
 #define DXMC_MAJORANT_CELL_MM 6.0
@@ -1097,6 +1097,7 @@ try {
     P.palette_index = w->palette_index;
     P.palette = w->palette;
     P.palette_n = static_cast<int>(palette.size());
+    P.has_measurement = d->measurement ? 1 : 0;
     for (int i = 0; i < 3; ++i) {
         P.dims[i] = static_cast<uint32_t>(d->dims[i]);
         P.inv_spacing[i] = static_cast<float>(1.0 / static_cast<double>(static_cast<float>(d->spacing[i])));
@@ -1212,17 +1213,14 @@ try {
     *bands = g->bands;
     for (int k = 0; band_edges && k + 1 < g->bands; ++k)
         band_edges[k] = g->band_edge[k];
-    cudaSetDevice(ctx->device);
-    cudaError_t e = cudaSuccess;
-    if (box)
-        e = cudaMemcpyAsync(box, g->box, 6 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && !cells)
-        e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess)
-        return cuda_fail(ctx, e, "local-majorant grid read");
+    for (int a = 0; box && a < 3; ++a) {
+        box[a] = g->box_lo[a];
+        box[3 + a] = g->box_hi[a];
+    }
     if (cells) {
         const uint64_t n = static_cast<uint64_t>(cells_per_axis[0]) * cells_per_axis[1] * cells_per_axis[2] * g->bands;
-        e = cudaMemcpyAsync(cells, g->cells, n * sizeof(float2), cudaMemcpyDeviceToHost, ctx->stream);
+        cudaSetDevice(ctx->device);
+        cudaError_t e = cudaMemcpyAsync(cells, g->cells, n * sizeof(float2), cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess)
             e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess)
@@ -1256,10 +1254,6 @@ try {
     off = align_up(off + static_cast<size_t>(nm) * R * 6, 4);
     m.off_maxcoef = static_cast<int>(off);
     off = align_up(off + static_cast<size_t>(R) * 2, 4);
-    m.off_rita = static_cast<int>(off);
-    off = align_up(off + static_cast<size_t>(nm) * 4 * dev::RITA_N, 4);
-    m.off_spline = static_cast<int>(off);
-    off = align_up(off + static_cast<size_t>(nm) * dev::SPLINE_FLOATS, 4);
     m.off_shells = static_cast<int>(off);
     off = align_up(off + static_cast<size_t>(nm) * dev::N_SHELLS * dev::SHELL_FLOATS, 4);
     m.total_floats = static_cast<int>(off);
@@ -1271,15 +1265,6 @@ try {
     for (int i = 0; i < R * 2; ++i)
         img[m.off_maxcoef + i] = static_cast<float>(b->max_coefficients[i]);
     for (int mat = 0; mat < nm; ++mat) {
-        for (int k = 0; k < 4 * dev::RITA_N; ++k)
-            img[m.off_rita + mat * 4 * dev::RITA_N + k] = static_cast<float>(b->rita[mat][k]);
-        float* sp = img.data() + m.off_spline + mat * dev::SPLINE_FLOATS;
-        for (int k = 0; k < 60; ++k)
-            sp[k] = static_cast<float>(b->spline[mat][k]);
-        sp[60] = static_cast<float>(b->spline[mat][76]);
-        sp[61] = static_cast<float>(b->spline[mat][77]);
-        sp[62] = static_cast<float>(b->spline[mat][78]);
-        sp[63] = static_cast<float>(1.0 / b->spline[mat][77]);
         for (int s = 0; s < dev::N_SHELLS; ++s) {
             const auto& c = b->shells[mat][s];
             float* o = img.data() + m.off_shells + (mat * dev::N_SHELLS + s) * dev::SHELL_FLOATS;
@@ -1515,7 +1500,7 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
             use_box = use_box || floor_level[band] >= 0;
         }
     }
-    const uint64_t cell_bytes = ncell * b.bands * sizeof(float2) + 8 * sizeof(float); // + the box
+    const uint64_t cell_bytes = ncell * b.bands * sizeof(float2);
     if (ctx->in_use + cell_bytes > ctx->budget)
         return fail(ctx, DXMC_ERR_OOM, "local-majorant grid exceeds the device memory budget");
     // least recently used first, never a grid the current submission reads
@@ -1536,13 +1521,15 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
     // returns, so jobs on any stream read it without a cross-stream wait
     cudaStream_t s = ctx->upload_stream;
     float2* cells = nullptr;
+    float* box = nullptr;
     uint8_t* level = nullptr;
     uint8_t* minlev = nullptr;
     float *d0 = nullptr, *d1 = nullptr, *cost = nullptr, *d_scales = nullptr;
     int* bounds = nullptr;
     unsigned int* d_hist = nullptr;
     cudaError_t e = pool_alloc(ctx, &cells, cell_bytes, s);
-    float* box = cells ? reinterpret_cast<float*>(cells + ncell * b.bands) : nullptr;
+    if (e == cudaSuccess)
+        e = pool_alloc(ctx, &box, 6 * sizeof(float), s);
     if (e == cudaSuccess)
         e = pool_alloc(ctx, &bounds, 6 * sizeof(int), s);
     if (e == cudaSuccess)
@@ -1653,12 +1640,13 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
         }
         e = dev::launch_majorant_level_passes(b, pg, minlev, d0, d1, cells, cost, s);
     }
-    static const float no_box[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
+    // the box goes into the kernels' parameters: read back with the wait that ends the build
+    float host_box[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
     if (e == cudaSuccess && use_box)
         e = dev::launch_majorant_box(b, bounds, cells, box, s);
-    else if (e == cudaSuccess) // an empty box: no cell is marked, the read-back says so
-        e = cudaMemcpyAsync(box, no_box, sizeof(no_box), cudaMemcpyHostToDevice, s);
-    for (void* ptr : { static_cast<void*>(level), static_cast<void*>(minlev), static_cast<void*>(d0), static_cast<void*>(d1), static_cast<void*>(cost),
+    if (e == cudaSuccess && use_box)
+        e = enqueue_readback(ctx, box, 0, sizeof(host_box), s);
+    for (void* ptr : { static_cast<void*>(box), static_cast<void*>(level), static_cast<void*>(minlev), static_cast<void*>(d0), static_cast<void*>(d1), static_cast<void*>(cost),
              static_cast<void*>(bounds), static_cast<void*>(d_scales), static_cast<void*>(d_hist) })
         if (ptr)
             cudaFreeAsync(ptr, s);
@@ -1670,6 +1658,8 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
         cudaStreamSynchronize(s);
         return cuda_fail(ctx, e, "local-majorant grid");
     }
+    if (use_box)
+        std::memcpy(host_box, ctx->readback_host, sizeof(host_box));
     MajorantCache m;
     m.lut_serial = lut->serial;
     m.cells = cells;
@@ -1677,7 +1667,10 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
     m.last_use = ++w->majorant_clock;
     m.submission = ctx->submission;
     m.grid.cells = cells;
-    m.grid.box = box;
+    for (int a = 0; a < 3; ++a) {
+        m.grid.box_lo[a] = host_box[a];
+        m.grid.box_hi[a] = host_box[3 + a];
+    }
     m.grid.nx = b.n[0];
     m.grid.nxy = b.n[0] * b.n[1];
     for (int a = 0; a < 3; ++a)
@@ -1933,7 +1926,7 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
     p.counters = j->counters;
     p.cancel = j->cancel_dev;
     p.total_histories = total;
-    p.seed = jd->seed;
+    p.stream_key = stream_key(jd->seed);
     p.tally_mode = tally_mode;
     p.precision = jd->precision;
     p.uniform_hpe = 0;
@@ -1991,24 +1984,25 @@ struct LaunchPlan {
 };
 
 // Grid, block and shared memory of a job's transport kernel; sets p.lut_in_smem.
-LaunchPlan plan_launch(dxmc_gpu_ctx* ctx, const dxmc_world* world, const dxmc_lut* lut, const dxmc_job_desc* jd, dev::TransportParams& p)
+LaunchPlan plan_launch(dxmc_gpu_ctx* ctx, const dxmc_lut* lut, const dxmc_job_desc* jd, bool queued, dev::TransportParams& p)
 {
     const int model = jd->model;
     LaunchPlan L;
-    const size_t lut_bytes = static_cast<size_t>(lut->meta.total_floats) * sizeof(float);
+    const size_t lut_bytes = static_cast<size_t>(dev::staged_lut_floats(lut->meta, model)) * sizeof(float);
     const size_t smem_limit = std::min<size_t>(ctx->max_smem_optin, 96 * 1024);
     p.lut_in_smem = lut_bytes <= smem_limit ? 1 : 0;
-    const bool palette = world->palette_index != nullptr;
-    L.smem = dev::transport_smem_bytes(lut_bytes, p.lut_in_smem != 0, palette);
+    const dev::TransportVariant variant = dev::transport_variant(p, model, queued);
+    L.smem = dev::transport_smem_bytes(variant, lut->meta, p.lut_in_smem != 0);
     L.block = jd->block_size == 128 || jd->block_size == 256 ? jd->block_size
-                                                              : (ctx->options.block_size > 0 ? ctx->options.block_size : 256);
+                                                              : (ctx->options.block_size > 0 ? ctx->options.block_size : dev::TRANSPORT_THREADS);
     // also sets the kernel's dynamic shared-memory limit for this launch
-    const int occ = dev::transport_max_blocks_per_sm(model, palette, L.block, L.smem, p.precision);
+    const int occ = dev::transport_max_blocks_per_sm(variant, L.block, L.smem);
     int per_sm = jd->blocks_per_sm > 0 ? std::min(jd->blocks_per_sm, std::max(occ, 1))
                                         : (ctx->options.blocks_per_sm > 0 ? ctx->options.blocks_per_sm : occ);
     if (per_sm <= 0)
         per_sm = 1;
     L.grid = ctx->sm_count * per_sm;
+    p.work = dev::transport_work_split(p.total_histories, static_cast<uint64_t>(L.grid) * (L.block / 32), queued);
     L.gen_grid = ctx->sm_count * 8;
     return L;
 }
@@ -2066,7 +2060,7 @@ try {
     const int rc = prepare_job(ctx, world, lut, jd, QueueMode::own, 0, &j, p, chunk);
     if (rc != DXMC_OK)
         return rc;
-    const LaunchPlan L = plan_launch(ctx, world, lut, jd, p);
+    const LaunchPlan L = plan_launch(ctx, lut, jd, chunk > 0, p);
     cudaError_t e = enqueue_job(j, p, jd->model, chunk, j->queue, L, ctx->stream, false);
     if (e == cudaSuccess)
         e = world->usage.mark(world->usage.on_stream, ctx->stream);
@@ -2489,7 +2483,7 @@ try {
         }
         std::vector<LaunchPlan> plans(n);
         for (int i = 0; i < n; ++i) // occupancy queries and attributes stay outside the capture
-            plans[i] = plan_launch(ctx, entries[i].world, entries[i].lut, entries[i].job, params[i]);
+            plans[i] = plan_launch(ctx, entries[i].lut, entries[i].job, chunks[i] > 0, params[i]);
         for (int c = 0; c < chains && e == cudaSuccess; ++c) {
             if (lists[c].empty())
                 continue;

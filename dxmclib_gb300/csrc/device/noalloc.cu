@@ -384,7 +384,7 @@ try {
         p.counters = reinterpret_cast<dev::JobCounters*>(s + OFF_COUNTERS);
         p.cancel = nullptr;
         p.total_histories = total;
-        p.seed = jd->seed;
+        p.stream_key = stream_key(jd->seed);
         p.tally_mode = 0; // FP64 atomics
         p.uniform_hpe = 0; // exposure found by binary search over the prefix sums
         // local majorants only from a grid built earlier (dxmc_gpu_world_prepare or a job)
@@ -396,15 +396,16 @@ try {
         p.regen_threshold = capi::ctx_regen_threshold(ctx, g != nullptr);
         p.interact_threshold = capi::ctx_interact_threshold(ctx);
         p.woodcock_burst = jd->woodcock_burst > 0 ? std::min(jd->woodcock_burst, 64) : capi::default_woodcock_burst(g != nullptr);
-        const size_t lut_bytes = static_cast<size_t>(meta.total_floats) * sizeof(float);
+        const size_t lut_bytes = static_cast<size_t>(dev::staged_lut_floats(meta, jd->model)) * sizeof(float);
         const size_t smem_limit = std::min<size_t>(capi::ctx_max_smem(ctx), 96 * 1024);
         p.lut_in_smem = lut_bytes <= smem_limit ? 1 : 0;
-        const bool palette = wp->palette_index != nullptr;
-        const size_t smem = dev::transport_smem_bytes(lut_bytes, p.lut_in_smem != 0, palette);
-        const int block = 256;
-        int per_sm = dev::transport_max_blocks_per_sm(jd->model, palette, block, smem, jd->precision);
+        const dev::TransportVariant variant = dev::transport_variant(p, jd->model, false);
+        const size_t smem = dev::transport_smem_bytes(variant, meta, p.lut_in_smem != 0);
+        const int block = dev::TRANSPORT_THREADS;
+        int per_sm = dev::transport_max_blocks_per_sm(variant, block, smem);
         if (per_sm <= 0)
             per_sm = 1;
+        p.work = dev::transport_work_split(total, static_cast<uint64_t>(capi::ctx_sm_count(ctx)) * per_sm * (block / 32), false);
         e = dev::launch_transport(p, jd->model, capi::ctx_sm_count(ctx) * per_sm, block, smem, stream);
     }
     // the counters are read back on every call (into this stack copy, no allocation):

@@ -51,9 +51,7 @@ struct LutMeta {
     int off_x;       // R log10 energies
     int off_coef;    // n_materials * R * 6
     int off_maxcoef; // R * 2
-    int off_rita;    // n_materials * 4 * 56 (x, e, a, b)
-    int off_spline;  // n_materials * 64 (60 coefficients, start, step, stop, pad)
-    int off_shells;  // n_materials * 12 * SHELL_FLOATS
+    int off_shells;  // n_materials * 12 * SHELL_FLOATS (read by the impulse-approximation model only)
     // inverse-CDF sampling tables, after total_floats (read from global memory,
     // not staged in shared memory): rows of tab_nu + 1 quantiles
     int off_ckn;     // Compton energy fraction, no scatter factor: tab_ne rows
@@ -137,9 +135,6 @@ __device__ __forceinline__ Real table_quantile(const float* row, int nu, Real u,
     return m_fma(fe, q1 - q0, q0);
 }
 
-constexpr int RITA_N = 56;
-constexpr int SPLINE_N = 16;
-constexpr int SPLINE_FLOATS = 64;
 constexpr int SHELL_FLOATS = 12; // binding, nElectrons, J0, photoProb, yield, lineP[3], lineE[3], pad
 constexpr int N_SHELLS = 12;
 
@@ -169,10 +164,11 @@ constexpr double N_ERROR_D = 1.0e-9;
 struct Rng {
     uint32_t s0, s1, s2, s3;
 
-    __device__ void init(uint64_t seed, uint64_t history)
+    __device__ void init(uint64_t seed, uint64_t history) { init_keyed(dxmc_gb300::stream_key(seed), history); }
+    __device__ void init_keyed(uint64_t key, uint64_t history)
     {
         uint32_t st[4];
-        stream_seed(seed, history, st);
+        stream_state(key, history, st);
         s0 = st[0];
         s1 = st[1];
         s2 = st[2];
@@ -191,6 +187,18 @@ struct Rng {
         s2 ^= t;
         s3 = __funnelshift_l(s3, s3, 11);
         return result;
+    }
+    // takes the last draw back (the state update of next() inverted)
+    __device__ __forceinline__ void step_back()
+    {
+        const uint32_t mixed = s1 ^ s2;                                  // s1 ^ (s1 << 9) of the earlier state
+        const uint32_t p1 = mixed ^ (mixed << 9) ^ (mixed << 18) ^ (mixed << 27);
+        const uint32_t t2 = s1 ^ p1;                                     // s2 ^ s0
+        const uint32_t t3 = __funnelshift_r(s3, s3, 11);                 // s3 ^ s1
+        s0 ^= t3;
+        s1 = p1;
+        s2 = t2 ^ s0;
+        s3 = t3 ^ p1;
     }
     // [0, 1) with 23 random bits: the top bits as the mantissa of a float in [1, 2),
     // minus one (no integer-to-float conversion)

@@ -34,18 +34,29 @@ DXMC_HD inline std::uint64_t splitmix64(std::uint64_t& x)
     return z ^ (z >> 31);
 }
 
-// The xoshiro128+ state of history `history` of a job seeded with `seed`; the
-// all-zero state is excluded by setting the lowest bit of the last word.
-DXMC_HD inline void stream_seed(std::uint64_t seed, std::uint64_t history, std::uint32_t out[4])
+// The job seed, mixed: the same for every history, so kernels take it ready-made.
+DXMC_HD inline std::uint64_t stream_key(std::uint64_t seed)
 {
     std::uint64_t k = seed;
-    std::uint64_t x = splitmix64(k) ^ history;
+    return splitmix64(k);
+}
+
+// The xoshiro128+ state of history `history` of the job with this stream key; the
+// all-zero state is excluded by setting the lowest bit of the last word.
+DXMC_HD inline void stream_state(std::uint64_t key, std::uint64_t history, std::uint32_t out[4])
+{
+    std::uint64_t x = key ^ history;
     const std::uint64_t a = splitmix64(x);
     const std::uint64_t b = splitmix64(x);
     out[0] = static_cast<std::uint32_t>(a);
     out[1] = static_cast<std::uint32_t>(a >> 32);
     out[2] = static_cast<std::uint32_t>(b);
     out[3] = static_cast<std::uint32_t>(b >> 32) | 1u;
+}
+
+DXMC_HD inline void stream_seed(std::uint64_t seed, std::uint64_t history, std::uint32_t out[4])
+{
+    stream_state(stream_key(seed), history, out);
 }
 
 DXMC_HD inline std::uint32_t mulhi32(std::uint32_t a, std::uint32_t b)

@@ -18,7 +18,7 @@ struct WorldParams {
     const uint8_t* palette_index;   // 1-byte layout, or nullptr when the world has > 256 distinct voxels
     const PaletteEntry* palette;    // PALETTE_MAX entries
     int palette_n;
-    int pad_palette;
+    int has_measurement;            // 1: the world has a measurement map (forced scoring)
     uint32_t dims[3];
     uint32_t pad;
     float lo[3];          // nextafter-safe lower extent (world.hpp:55-68)
@@ -48,7 +48,7 @@ struct WorldParams {
 constexpr int MAJORANT_MAX_BANDS = 8;
 struct MajorantGrid {
     const float2* cells;
-    const float* box;    // lo[3], hi[3] in mm (grid frame) of the cells above the emptiest level
+    float box_lo[3], box_hi[3]; // mm (grid frame), of the cells above the emptiest level; empty (lo > hi): no cell is marked
     uint32_t nx, nxy;    // cells along x, cells per z slab
     int shift[3];        // log2 of the cell size in voxels
     int bands;
@@ -108,6 +108,14 @@ struct alignas(32) TallyRecord {
 };
 static_assert(sizeof(TallyRecord) == 32, "one tally record per 32-byte sector");
 
+// A job's ids in units that a warp takes at a time: `large_units` of `large` ids, then
+// units of `small` (both multiples of 32).
+struct WorkSplit {
+    uint64_t large_units = 0;
+    uint32_t large = 256;
+    uint32_t small = 32;
+};
+
 struct TransportParams {
     WorldParams world;
     SourceParams source;
@@ -121,7 +129,7 @@ struct TransportParams {
     const volatile int* cancel; // host-mapped flag, may be null
     PhotonQueue queue;          // pos_energy == nullptr: photons are generated inside the transport kernel
     uint64_t total_histories;
-    uint64_t seed;
+    uint64_t stream_key;    // the job seed, mixed once (stream_key in stream_seed.hpp)
     uint64_t uniform_hpe;   // histories per exposure when every exposure has the same count, else 0
     uint32_t hpe_magic;     // history / uniform_hpe as a multiply-high (udiv_magic), jobs below 2^32 histories
     uint32_t hpe_shifts;
@@ -133,6 +141,7 @@ struct TransportParams {
     int normalize_direction; // 1: unit scattering axis in peturb (normalised physics), 0: the reference's
     int precision;          // 0: FP32 transport; 1: FP64 everywhere (position, direction, energy, LUT, sampling)
     int pad_precision;
+    WorkSplit work;         // how the warps share the histories (or queued photons)
     MajorantGrid majorant;
 };
 
@@ -172,10 +181,42 @@ cudaError_t launch_transport(const TransportParams& p, int model, int grid, int 
 // Loads the modules of every single-job transport kernel on the current device
 // (CUDA loads modules lazily, on first use, and a load allocates device memory).
 cudaError_t preload_transport_kernels();
+// Which single-job kernel a job runs.
+struct TransportVariant {
+    int model = 1;
+    int precision = 0;    // 1: FP64 everywhere
+    bool palette = false; // compact voxel layout
+    bool forced = true;   // forced photoelectric scoring (a measurement map)
+    // The options of nearly every job: FP32 transport with the FP64 record tally (mode 0),
+    // local majorants, photons sampled in the kernel, the reference's directions, and a LUT
+    // of at most ATT_TABLE_MATERIALS materials staged in shared memory.  Compiled apart,
+    // the kernel tests none of these in its loop and keeps a per-lane attenuation table.
+    bool fast = false;
+};
+// The attenuation table of the fast kernels: one float per material and lane of a block.
+// Eight materials cover the usual segmentations (the workloads use one to four)
+// in 1 KB per warp; filling a column costs about 20 instructions per material
+// when a photon's energy changes, which beyond eight exceeds what it saves.
+constexpr int ATT_TABLE_MATERIALS = 8;
+constexpr int TRANSPORT_THREADS = 256; // largest block of the single-job kernels
+// The part of the LUT image a kernel stages in shared memory.
+inline int staged_lut_floats(const LutMeta& m, int model) { return model == 2 ? m.total_floats : m.off_shells; }
+constexpr int ATT_TABLE_LANES = TRANSPORT_THREADS;
+// Each warp starts with the unit of its own number and fetches further ones from the
+// queue's counter, one address that serves 1.7 ns per fetch (fetching 32 histories at a
+// time, a job of 2e6 spent 0.1 of its 0.48 ms there).  Jobs of up to 24 rounds of 32
+// histories per warp give three quarters to the first units and even out what warps
+// differ by in units of 32; larger jobs fetch 256 at a time, in order, so that the
+// photons in flight stay within a few exposures and their voxels and tallies in L2
+// (interleaving the whole job statically took the CT workload from 12.6 to 14.3 ms),
+// and the last six rounds 64 at a time.
+WorkSplit transport_work_split(uint64_t histories, uint64_t warps, bool queued);
+// (queued: photons come from the pre-generated queue)
+TransportVariant transport_variant(const TransportParams& p, int model, bool queued);
 // blocks per SM for this configuration; also raises the kernel's dynamic shared-memory limit
-int transport_max_blocks_per_sm(int model, bool palette, int block, size_t smem, int precision = 0);
-// dynamic shared memory the transport kernel needs for a LUT image of lut_bytes
-size_t transport_smem_bytes(size_t lut_bytes, bool lut_in_smem, bool palette);
+int transport_max_blocks_per_sm(const TransportVariant& v, int block, size_t smem);
+// dynamic shared memory the transport kernel needs
+size_t transport_smem_bytes(const TransportVariant& v, const LutMeta& meta, bool lut_in_smem);
 // Post-processing of the tallies into dose / variance (densities from the world's layout).
 // dose, variance and counts_out may be device memory or page-locked host memory
 // (written through its device mapping); counts_out, if not null, gets a copy of counts.

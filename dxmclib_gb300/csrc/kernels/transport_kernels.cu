@@ -9,16 +9,15 @@
 // device function names the reference lines it restates.
 #include "transport.cuh"
 
-#include <mutex>
-
 #include <algorithm>
+#include <mutex>
+#include <unordered_map>
 
 namespace dxmc_gb300::dev {
 
 namespace {
 
     constexpr unsigned FULL_MASK = 0xffffffffu;
-    constexpr int WARP_POOL_CHUNK = 256; // histories fetched per queue access
     constexpr uint32_t MAX_STEPS_PER_HISTORY = 1u << 20; // guard against unbounded histories
 
     template <class Real>
@@ -33,39 +32,30 @@ namespace {
     // Atomic additions to the tally with an L2 evict-first policy: the tally is
     // read-modify-written at random voxels and would otherwise push the voxel and
     // majorant grids (gathered on every flight) out of L2.
-    __device__ __forceinline__ void red_add_evict_first(double* a, double v)
-    {
-#ifdef DXMC_TALLY_NO_HINT
-        atomicAdd(a, v);
-        return;
-#endif
-        asm volatile("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
-                     "red.global.add.L2::cache_hint.f64 [%0], %1, pol;\n\t}" ::"l"(a), "d"(v) : "memory");
-    }
-    __device__ __forceinline__ void red_add_evict_first(uint32_t* a, uint32_t v)
-    {
-#ifdef DXMC_TALLY_NO_HINT
-        atomicAdd(a, v);
-        return;
-#endif
-        asm volatile("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
-                     "red.global.add.L2::cache_hint.u32 [%0], %1, pol;\n\t}" ::"l"(a), "r"(v) : "memory");
-    }
     __device__ __forceinline__ void score_record(TallyRecord* r, double e, double e2, uint32_t n)
     {
-        red_add_evict_first(&r->energy, e);
-        red_add_evict_first(&r->energy2, e2);
-        red_add_evict_first(&r->events, n);
+#ifdef DXMC_TALLY_NO_HINT
+        atomicAdd(&r->energy, e);
+        atomicAdd(&r->energy2, e2);
+        atomicAdd(&r->events, n);
+#else
+        asm volatile("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
+                     "red.global.add.L2::cache_hint.f64 [%0], %1, pol;\n\t"
+                     "red.global.add.L2::cache_hint.f64 [%0+8], %2, pol;\n\t"
+                     "red.global.add.L2::cache_hint.u32 [%0+16], %3, pol;\n\t}" ::"l"(r), "d"(e), "d"(e2), "r"(n) : "memory");
+#endif
     }
 
-    template <class Real>
+    template <bool FAST, class Real>
     __device__ __forceinline__ void score(const TransportParams& p, uint64_t idx, Real e)
     {
-        if (p.records) {
+        if (FAST || p.records) {
             const double ed = static_cast<double>(e);
             score_record(p.records + idx, ed, ed * ed, 1u);
             return;
         }
+        if constexpr (FAST)
+            return;
         if (p.tally_mode == 1) {
             float* t = p.tally_f32 + 2 * idx;
             atomicAdd(t, e);
@@ -110,30 +100,52 @@ namespace {
         }
     }
 
-    // ---- photoelectric (transport.hpp:216-263) ---------------------------------
-    template <int MODEL, class Real>
-    __device__ __forceinline__ Real photo_absorption(const float* L, const LutMeta& m, PhotonT<Real>& ph, int material, Rng& rng, bool norm = false)
+    // Sums and products that the compiler must not fuse: its choice would change with the
+    // code around them, and the last bit of a history with it.
+    __device__ __forceinline__ float add_rounded(float a, float b) { return __fadd_rn(a, b); }
+    __device__ __forceinline__ double add_rounded(double a, double b) { return __dadd_rn(a, b); }
+    __device__ __forceinline__ float mul_rounded(float a, float b) { return __fmul_rn(a, b); }
+    __device__ __forceinline__ double mul_rounded(double a, double b) { return __dmul_rn(a, b); }
+
+    // The samplers below draw an interaction's outcome (energy imparted, new energy,
+    // cosine of the scattering angle); the direction changes in one place for all of
+    // them, by an azimuth drawn last (peturb).
+
+    // Shell of a photoelectric or impulse-approximation Compton event: the first
+    // whose cumulated weight reaches u times the total.  The partial sums are taken
+    // in the same order for the total and for the search, so both use one list.
+    template <class Real>
+    __device__ __forceinline__ int pick_shell(const Real (&cum)[N_SHELLS], Real u)
     {
-        const Real E = ph.energy;
-        ph.energy = Real(0.0);
+        const Real sample = cum[N_SHELLS - 1] * u;
+        int idx = 0;
+#pragma unroll
+        for (int s = 0; s < N_SHELLS - 1; ++s)
+            idx += cum[s] < sample ? 1 : 0; // the sums do not decrease
+        return idx;
+    }
+
+    // ---- photoelectric (transport.hpp:216-263) ---------------------------------
+    // Returns the energy imparted; `turn`: a characteristic photon of `energy` leaves
+    // at angle cosA, otherwise energy is 0.
+    template <int MODEL, class Real>
+    __device__ __forceinline__ Real photo_sample(const float* L, const LutMeta& m, Real& energy, int material, Rng& rng, Real& cosA, bool& turn)
+    {
+        const Real E = energy;
+        energy = Real(0.0);
+        turn = false;
         if constexpr (MODEL < 2) {
             return E;
         } else {
             const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
+            Real cum[N_SHELLS];
             Real total = Real(0.0);
 #pragma unroll
-            for (int s = 0; s < N_SHELLS; ++s)
-                total += E > shells[s * SHELL_FLOATS] ? shells[s * SHELL_FLOATS + 3] : Real(0.0);
-            const Real sample = total * static_cast<Real>(rng.uniform());
-            Real cum = Real(0.0);
-            int idx = 0;
             for (int s = 0; s < N_SHELLS; ++s) {
-                cum += E > shells[s * SHELL_FLOATS] ? shells[s * SHELL_FLOATS + 3] : Real(0.0);
-                idx = s;
-                if (!(cum < sample) || s == N_SHELLS - 1)
-                    break;
+                total += E > shells[s * SHELL_FLOATS] ? shells[s * SHELL_FLOATS + 3] : Real(0.0);
+                cum[s] = total;
             }
-            const float* sh = shells + idx * SHELL_FLOATS;
+            const float* sh = shells + pick_shell(cum, static_cast<Real>(rng.uniform())) * SHELL_FLOATS;
             const Real binding = sh[0];
             if (binding > E || binding < Real(ENERGY_CUTOFF_D))
                 return E;
@@ -145,19 +157,33 @@ namespace {
                     ++line;
                     r3 -= sh[5 + line];
                 }
-                ph.energy = sh[8 + line];
+                energy = sh[8 + line];
                 const Real theta = static_cast<Real>(rng.uniform()) * Real(PI_D);
-                const Real phi = rng_azimuth<Real>(rng);
-                peturb(ph.dx, ph.dy, ph.dz, m_cos(theta), phi, norm);
-                return E - ph.energy;
+                cosA = m_cos(theta);
+                turn = true;
+                return E - energy;
             }
             return E;
         }
     }
 
+    // The whole photoelectric event on a photon, direction included.
+    template <int MODEL, class Real>
+    __device__ __forceinline__ Real photo_absorption(const float* L, const LutMeta& m, PhotonT<Real>& ph, int material, Rng& rng, bool norm = false)
+    {
+        Real cosA = Real(1.0);
+        bool turn;
+        const Real imparted = photo_sample<MODEL>(L, m, ph.energy, material, rng, cosA, turn);
+        if (turn) {
+            const Real phi = rng_azimuth<Real>(rng);
+            peturb(ph.dx, ph.dy, ph.dz, cosA, phi, norm);
+        }
+        return imparted;
+    }
+
     // ---- Rayleigh (transport.hpp:264-298) ---------------------------------------
     template <int MODEL, class Real>
-    __device__ __forceinline__ bool rayleigh_scatter(const float* L, const float* G, const LutMeta& m, PhotonT<Real>& ph, int material, Rng& rng, bool norm = false)
+    __device__ __forceinline__ bool rayleigh_sample(const float* G, const LutMeta& m, Real energy, int material, Rng& rng, Real& cosA)
     {
         if constexpr (MODEL == 0) {
             constexpr Real extreme = Real(1.08866210790363); // 4 sqrt(2) / (3 sqrt(3))
@@ -167,8 +193,7 @@ namespace {
                 Real s, c;
                 m_sincos(theta, &s, &c);
                 if (!(r1 > (Real(2.0) - s * s) * s)) {
-                    const Real phi = rng_azimuth<Real>(rng);
-                    peturb(ph.dx, ph.dy, ph.dz, c, phi, norm);
+                    cosA = c;
                     return true;
                 }
             }
@@ -177,52 +202,47 @@ namespace {
             // the density of the reference's RITA draw of q^2 <= q_max^2 followed by the
             // (1 + cos^2) / 2 rejection, drawn by inverse CDF: no loop, no divergence
             Real fe;
-            const int row = table_row(m, ph.energy, fe);
+            const int row = table_row(m, energy, fe);
             const Real y = table_quantile(G + m.off_ray + (material * m.tab_ne + row) * (m.tab_nu + 1), m.tab_nu, static_cast<Real>(rng.uniform()), fe);
-            const Real cosA = Real(1.0) - Real(2.0) * y; // q^2 / q_max^2 = (1 - cos) / 2
-            const Real phi = rng_azimuth<Real>(rng);
-            peturb(ph.dx, ph.dy, ph.dz, cosA, phi, norm);
+            cosA = Real(1.0) - Real(2.0) * y; // q^2 / q_max^2 = (1 - cos) / 2
             return true;
         }
     }
 
     // ---- Compton, impulse approximation (transport.hpp:342-483) -----------------
+    // The electron shell that takes part, or -1 where the interaction is rejected
+    // (no shell can take part, or its binding energy exceeds the photon's).
     template <class Real>
-    __device__ __forceinline__ bool compton_ia(const float* L, const LutMeta& m, PhotonT<Real>& ph, int material, Rng& rng, Real& deposit, bool norm = false)
+    __device__ __forceinline__ int compton_shell(const float* L, const LutMeta& m, Real energy, int material, Rng& rng)
     {
         const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
+        Real cum[N_SHELLS];
         Real total = Real(0.0);
 #pragma unroll
-        for (int s = 0; s < N_SHELLS; ++s)
-            total += (shells[s * SHELL_FLOATS] < ph.energy && shells[s * SHELL_FLOATS + 2] > Real(0.0)) ? shells[s * SHELL_FLOATS + 1] : Real(0.0);
-        const Real sample = total * static_cast<Real>(rng.uniform());
-        Real cum = Real(0.0);
-        int shell = 0;
         for (int s = 0; s < N_SHELLS; ++s) {
-            cum += (shells[s * SHELL_FLOATS] < ph.energy && shells[s * SHELL_FLOATS + 2] > Real(0.0)) ? shells[s * SHELL_FLOATS + 1] : Real(0.0);
-            shell = s;
-            if (!(cum < sample) || s == N_SHELLS - 1)
-                break;
+            total += (shells[s * SHELL_FLOATS] < energy && shells[s * SHELL_FLOATS + 2] > Real(0.0)) ? shells[s * SHELL_FLOATS + 1] : Real(0.0);
+            cum[s] = total;
         }
-        if (!(total > Real(0.0))) {
-            deposit = Real(0.0); // no shell can take part: the interaction is rejected
-            return true;
-        }
-        const float* sh = shells + shell * SHELL_FLOATS;
+        const int shell = pick_shell(cum, static_cast<Real>(rng.uniform()));
+        if (!(total > Real(0.0)))
+            return -1;
+        const Real U = shells[shell * SHELL_FLOATS] / Real(ELECTRON_REST_MASS_D);
+        return U > energy / Real(ELECTRON_REST_MASS_D) ? -1 : shell; // the rejection corrects the cross section
+    }
+
+    // Energy fraction e and angle of a Compton event with shell `sh` by rejection.
+    template <class Real>
+    __device__ __forceinline__ bool compton_ia(const float* sh, Real energy, Rng& rng, Real& e, Real& cosA)
+    {
         const Real U = sh[0] / Real(ELECTRON_REST_MASS_D);
         const Real pU = m_sqrt(Real(2.0) * U + U * U);
         const Real J0 = sh[2];
-        const Real k = ph.energy / Real(ELECTRON_REST_MASS_D);
-        if (U > k) {
-            deposit = Real(0.0); // interaction rejected (corrects the cross section)
-            return true;
-        }
+        const Real k = energy / Real(ELECTRON_REST_MASS_D);
         const Real emin = Real(1.0) / (Real(1.0) + Real(2.0) * k);
         const Real gmax_inv = Real(1.0) / (Real(1.0) / emin + emin);
         constexpr Real sp2 = Real(2.50662827463100); // 1 / (1/sqrt(pi) / sqrt(2)) = sqrt(2 pi)
         constexpr Real a1 = Real(0.34802), a2 = -Real(0.0958798), a3 = Real(0.7478556);
         const Real sqrte = Real(1.64872127070013);
-        Real e = Real(1.0), cosA = Real(1.0);
         bool accepted = false;
         for (int it = 0; it < REJECTION_CAP && !accepted; ++it) {
             const Real r1 = static_cast<Real>(rng.uniform());
@@ -237,7 +257,10 @@ namespace {
             const Real r2 = static_cast<Real>(rng.uniform());
             if (r2 > g)
                 continue;
-            const Real pi = (k * (k - U) * t - U) / m_sqrt(m_max(Real(2.0) * k * (k - U) * t + U * U, Real(1e-30)));
+            // the product is rounded where the second term takes it, as a rule written out:
+            // pi is a difference of near numbers for small angles
+            const Real kU = k * (k - U);
+            const Real pi = m_fma(kU, t, -U) / m_sqrt(m_max(m_fma(U, U, Real(2.0) * mul_rounded(kU, t)), Real(1e-30)));
             const Real kc = k * e;
             const Real qc = m_sqrt(m_max(k * k + kc * kc - Real(2.0) * k * kc * cosA, Real(1e-30)));
             const Real alpha = qc * (Real(1.0) + kc * (kc - k * cosA) / (qc * qc)) / k;
@@ -295,42 +318,53 @@ namespace {
             e = kbar / k;
             accepted = true;
         }
-        if (!accepted)
-            return false;
-        const Real phi = rng_azimuth<Real>(rng);
-        peturb(ph.dx, ph.dy, ph.dz, cosA, phi, norm);
-        const Real E = ph.energy;
-        ph.energy *= e;
-        deposit = E - ph.energy;
-        return true;
+        return accepted;
     }
 
     // ---- Compton, Klein-Nishina with optional scatter factor (transport.hpp:300-340)
-    template <int MODEL, class Real>
-    __device__ __forceinline__ bool compton_scatter(const float* L, const float* G, const LutMeta& m, PhotonT<Real>& ph, int material, Rng& rng, Real& deposit, bool norm = false)
+    // Energy fraction and angle from the quantile x = (e - e_min) / (1 - e_min).
+    template <class Real>
+    __device__ __forceinline__ void compton_from_fraction(Real E, Real x, Real& e, Real& cosA)
     {
+        const Real k = E / Real(ELECTRON_REST_MASS_D);
+        const Real emin = Real(1.0) / (Real(1.0) + Real(2.0) * k);
+        const Real one_minus_e = (Real(1.0) - x) * (Real(1.0) - emin);
+        e = Real(1.0) - one_minus_e;
+        cosA = m_max(Real(1.0) - one_minus_e / (k * e), -Real(1.0));
+    }
+
+    // Returns false where the sampling loop hit its cap; `turn` false: the interaction
+    // was rejected (nothing changes, zero energy imparted).
+    template <int MODEL, class Real>
+    __device__ __forceinline__ bool compton_sample(const float* L, const float* G, const LutMeta& m, Real& energy, int material, Rng& rng, Real& cosA,
+        Real& imparted, bool& turn)
+    {
+        const Real E = energy;
+        imparted = Real(0.0);
+        turn = true;
+        Real e;
         if constexpr (MODEL == 2) {
-            return compton_ia(L, m, ph, material, rng, deposit, norm);
+            const int shell = compton_shell(L, m, E, material, rng);
+            if (shell < 0) {
+                turn = false;
+                return true;
+            }
+            e = Real(1.0);
+            if (!compton_ia(L + m.off_shells + (material * N_SHELLS + shell) * SHELL_FLOATS, E, rng, e, cosA))
+                return false;
         } else {
             // the density of the reference's Klein-Nishina rejection (times the scatter
             // factor S(q) for LIVERMORE), drawn by inverse CDF: no loop, no divergence
-            const Real E = ph.energy;
-            const Real k = E / Real(ELECTRON_REST_MASS_D);
-            const Real emin = Real(1.0) / (Real(1.0) + Real(2.0) * k);
             Real fe;
             const int row = table_row(m, E, fe);
             const float* tab = MODEL == 1 ? G + m.off_csf + (material * m.tab_ne + row) * (m.tab_nu + 1)
                                           : G + m.off_ckn + row * (m.tab_nu + 1);
-            const Real x = table_quantile(tab, m.tab_nu, static_cast<Real>(rng.uniform()), fe); // (e - e_min) / (1 - e_min)
-            const Real one_minus_e = (Real(1.0) - x) * (Real(1.0) - emin);
-            const Real e = Real(1.0) - one_minus_e;
-            const Real cosA = Real(1.0) - one_minus_e / (k * e);
-            const Real phi = rng_azimuth<Real>(rng);
-            peturb(ph.dx, ph.dy, ph.dz, m_max(cosA, -Real(1.0)), phi, norm);
-            ph.energy = E * e;
-            deposit = E - ph.energy;
-            return true;
+            const Real x = table_quantile(tab, m.tab_nu, static_cast<Real>(rng.uniform()), fe);
+            compton_from_fraction(E, x, e, cosA);
         }
+        energy = E * e;
+        imparted = E - energy;
+        return true;
     }
 
     // ---- photon generation: Exposure::sampleParticle (exposure.hpp:280-304) -----
@@ -472,31 +506,33 @@ namespace {
             dst[i] = __ldg(src + i);
     }
 
-    // ---- the transport kernel ----------------------------------------------------
-    //
-    // Warp-synchronous loop.  Each iteration every lane with a live photon and no
-    // pending interaction takes up to woodcock_burst Woodcock steps; a real event
-    // only records its type (photoelectric / Compton / Rayleigh) and ends the lane's
-    // burst.  The interactions are then run in
-    // one converged pass per type once enough lanes wait, and finished lanes are
-    // refilled together once enough are idle, so the expensive branches run with
-    // many lanes active instead of one or two.
-    enum : int { EV_NONE = 0, EV_PHOTO = 1, EV_COMPTON = 2, EV_RAYLEIGH = 3 };
-
     // A voxel as read from the grid: its palette index (compact layout) or its
     // 8-byte record; decode_voxel turns it into density, material and the
-    // measurement flag.
+    // measurement flag.  Compact worlds hold fewer than 2^32 voxels (world upload),
+    // so their voxel index is 32 bits.
     template <bool PALETTE>
     struct VoxelRaw {
+        using Index = uint64_t;
         uint2 v;
     };
     template <>
     struct VoxelRaw<true> {
+        using Index = uint32_t;
         uint32_t index;
     };
 
     template <bool PALETTE>
-    __device__ __forceinline__ VoxelRaw<PALETTE> load_voxel(const WorldParams& w, uint64_t vidx)
+    __device__ __forceinline__ typename VoxelRaw<PALETTE>::Index voxel_index(const WorldParams& w, uint32_t ix, uint32_t iy, uint32_t iz)
+    {
+        using Index = typename VoxelRaw<PALETTE>::Index;
+        if constexpr (PALETTE)
+            return iz * static_cast<uint32_t>(w.nxy) + (iy * w.dims[0] + ix);
+        else
+            return static_cast<Index>(iz) * w.nxy + static_cast<Index>(iy) * w.dims[0] + ix;
+    }
+
+    template <bool PALETTE>
+    __device__ __forceinline__ VoxelRaw<PALETTE> load_voxel(const WorldParams& w, typename VoxelRaw<PALETTE>::Index vidx)
     {
         if constexpr (PALETTE)
             return VoxelRaw<true> { __ldg(w.palette_index + vidx) };
@@ -519,46 +555,77 @@ namespace {
         }
     }
 
-#ifndef DXMC_RAYLEIGH_THRESHOLD
-#define DXMC_RAYLEIGH_THRESHOLD 2 // lanes waiting for a Rayleigh event before its pass runs alone
-#endif
-    constexpr int RAYLEIGH_THRESHOLD = DXMC_RAYLEIGH_THRESHOLD;
-
 #ifndef DXMC_MIN_BLOCKS_PER_SM
 #define DXMC_MIN_BLOCKS_PER_SM 4 // resident 256-thread blocks per SM the register budget must allow (64 registers)
 #endif
 
-    // State of one lane: its photon, random stream, cached lookups and counters.
-    // Per-warp counters of a job in shared memory (lane 0 adds warp totals; rare
-    // events use shared atomics), flushed to the job's counters: they cost the
-    // lanes no registers.
-    struct WarpTally {
-        unsigned long long steps, deposits, overflows, histories;
+    // Lanes that must still fly for a burst to go on: a further flight costs the warp
+    // about 100 instructions whatever its lanes, the loop's other stages about 700.
+    constexpr int MIN_FLYING = 5;
+
+    // What belongs to a warp rather than to a lane, in shared memory: in registers every
+    // lane would hold a copy through the whole loop (a dozen of its 64).
+    struct WarpState {
+        uint64_t next, end;                      // ids [next, end) to sample
+        int pooled;                              // photons in the pool
+        uint32_t steps, deposits, histories;     // since they were last added to the job's counters
+        unsigned int overflows, forced_deposits; // rare events, by shared atomics
     };
 
-    template <class Real>
+    // Adds the warp's counters to the job's and clears them (32 bits last for far longer
+    // than the 256 histories between two calls).  Called by all 32 lanes.
+    __device__ __forceinline__ void add_counters(WarpState& ws, JobCounters* c)
+    {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) {
+            if (ws.steps)
+                atomicAdd(&c->steps, static_cast<unsigned long long>(ws.steps));
+            if (ws.deposits + ws.forced_deposits)
+                atomicAdd(&c->deposits, static_cast<unsigned long long>(ws.deposits) + ws.forced_deposits);
+            if (ws.overflows)
+                atomicAdd(&c->overflows, static_cast<unsigned long long>(ws.overflows));
+            if (ws.histories)
+                atomicAdd(&c->histories_done, static_cast<unsigned long long>(ws.histories));
+            ws.steps = ws.deposits = ws.histories = 0;
+            ws.overflows = ws.forced_deposits = 0;
+        }
+        __syncwarp();
+    }
+
+    // What a lane does: it flies, it waits for a stage of the loop, or it waits for the
+    // event of a real collision in the material |state| - 1 (negative: at a forced-scoring
+    // voxel).  The event's type is drawn in the interaction pass, where more lanes share
+    // the work than in the flight loop.
+    constexpr int FLYING = 0;
+    constexpr int IDLE = 0x200;  // no photon
+    constexpr int SETUP = 0x201; // new photon or energy: majorant, attenuation and cell to look up
+    constexpr int REACH = 0x202; // the next flight leaves the ball of its cell outside the body box
+
+    __device__ __forceinline__ bool waits_for_event(int state) { return state != FLYING && state < IDLE; }
+
+    // State of one lane: its photon, random stream and cached lookups.
+    template <class Real, class Index>
     struct LaneT {
         PhotonT<Real> ph;
         Rng rng;
-        bool alive;
-        int pending;
-        Real stepK, logE; // Woodcock step = -log2(u) * stepK (mm): 10 * ln 2 / majorant
-        int seg;
-        bool updateMax;
-        int cached_mat;
+        int state;
+        Real stepK; // Woodcock step = -log2(u) * stepK (mm): 10 * ln 2 / majorant
         uint32_t hist_steps;
-        Real probInv;  // attenuation of the current material / majorant (event probability per unit density)
-        Real p0, p01;  // photoelectric and photoelectric + Compton shares of the attenuation
-        uint64_t vidx;
-        Real forced_wc; // weight correction waiting for a forced-voxel interaction pass
+        Index vidx;
         bool armed;      // energy x weight is below the Russian-roulette threshold
         Real cinv, cR;  // local majorant: 1 / scale and the flight length it holds for (MajorantGrid)
         int band;        // energy band of the local-majorant grid
+        // without the attenuation table: the last material met at this energy
+        Real logE;
+        int seg;
+        int cached_mat;
+        Real probInv;   // attenuation of the material / majorant (event probability per unit density)
+        Real p0, p01;   // FP64: photoelectric and photoelectric + Compton shares of the attenuation
+        Real forced_wc; // weight correction waiting for a forced-voxel interaction pass
 
         __device__ void start_photon()
         {
-            pending = EV_NONE;
-            updateMax = true;
+            state = SETUP;
             cached_mat = -1;
             hist_steps = 0;
             forced_wc = Real(0.0);
@@ -575,14 +642,14 @@ namespace {
     // changed (a new photon, or an interaction): the flight drawn next must be
     // bounded for the new energy.  A new photon sits on the grid boundary, so the
     // coordinates are clamped onto the grid.
-    template <class Real>
-    __device__ __forceinline__ void fetch_cell(LaneT<Real>& s, const TransportParams& p)
+    template <class Real, class Index>
+    __device__ __forceinline__ void fetch_cell(LaneT<Real, Index>& s, const TransportParams& p, Real logE)
     {
         const MajorantGrid& g = p.majorant;
         const WorldParams& w = p.world;
-        // s.logE = log10 E was just computed; the band intervals of the bounds are
-        // widened by 0.1 % on the host, which covers the rounding here
-        s.band = min(max(m_floor_int((s.logE - g.band_log0) * g.band_inv_dlog), 0), g.bands - 1);
+        // the band intervals of the bounds are widened by 0.1 % on the host, which
+        // covers the rounding here
+        s.band = min(max(m_floor_int((logE - g.band_log0) * g.band_inv_dlog), 0), g.bands - 1);
         const Real fx = m_min(m_max(m_fma(s.ph.px, w.inv_spacing[0], -w.lo_inv[0]), Real(0.0)), w.dims_f[0] - Real(1.0));
         const Real fy = m_min(m_max(m_fma(s.ph.py, w.inv_spacing[1], -w.lo_inv[1]), Real(0.0)), w.dims_f[1] - Real(1.0));
         const Real fz = m_min(m_max(m_fma(s.ph.pz, w.inv_spacing[2], -w.lo_inv[2]), Real(0.0)), w.dims_f[2] - Real(1.0));
@@ -606,8 +673,8 @@ namespace {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const Real inv = Real(1.0) / d[a];
-            const Real t0 = (__ldg(g.box + a) - p[a]) * inv;
-            const Real t1 = (__ldg(g.box + 3 + a) - p[a]) * inv;
+            const Real t0 = (g.box_lo[a] - p[a]) * inv;
+            const Real t1 = (g.box_hi[a] - p[a]) * inv;
             tmin = m_max(tmin, m_min(t0, t1));
             tmax = m_min(tmax, m_max(t0, t1));
         }
@@ -616,25 +683,24 @@ namespace {
 
     // Loads photon + stream state from the pre-generated queue.
     template <class Real>
-    __device__ __forceinline__ void take_queued(LaneT<Real>& s, const PhotonQueue& q, uint64_t i)
+    __device__ __forceinline__ void load_queued(PhotonT<Real>& ph, Rng& rng, const PhotonQueue& q, uint64_t i)
     {
         const float4 pe = __ldg(q.pos_energy + i);
         const float4 dw = __ldg(q.dir_weight + i);
         const uint4 rs = __ldg(q.rng + i);
-        s.ph = PhotonT<Real> { pe.x, pe.y, pe.z, dw.x, dw.y, dw.z, pe.w, dw.w };
-        s.rng.s0 = rs.x;
-        s.rng.s1 = rs.y;
-        s.rng.s2 = rs.z;
-        s.rng.s3 = rs.w;
-        s.alive = true;
-        s.start_photon();
+        ph = PhotonT<Real> { pe.x, pe.y, pe.z, dw.x, dw.y, dw.z, pe.w, dw.w };
+        rng.s0 = rs.x;
+        rng.s1 = rs.y;
+        rng.s2 = rs.z;
+        rng.s3 = rs.w;
     }
 
-    // Samples history h of the job in place (Exposure::sampleParticle + transportParticleToWorld).
+    // Samples history h of the job (Exposure::sampleParticle); false: it misses the
+    // grid (transportParticleToWorld).
     template <class Real>
-    __device__ __forceinline__ void take_history(LaneT<Real>& s, const TransportParams& p, uint64_t h)
+    __device__ __forceinline__ bool sample_history(PhotonT<Real>& ph, Rng& rng, const TransportParams& p, uint64_t h)
     {
-        s.rng.init(p.seed, h);
+        rng.init_keyed(p.stream_key, h);
         uint32_t ei;
         if (p.uniform_hpe && p.total_histories <= 0xffffffffull)
             ei = udiv_apply(static_cast<uint32_t>(h), p.hpe_magic, p.hpe_shifts);
@@ -642,364 +708,436 @@ namespace {
             ei = p.uniform_hpe ? static_cast<uint32_t>(h / p.uniform_hpe) : find_exposure(p.source, h);
         DevExposure ex;
         load_exposure(p.source.exposures + ei, ex);
-        sample_particle(p.source, ex, s.rng, s.ph);
-        s.alive = transport_to_world(p.world, s.ph);
-        s.start_photon();
+        sample_particle(p.source, ex, rng, ph);
+        return transport_to_world(p.world, ph);
     }
 
-    // One iteration of the warp-synchronous loop for every lane of the warp: a
-    // Woodcock step for lanes without a pending interaction (transport.hpp:650-699),
-    // the per-type interaction passes once enough lanes wait (transport.hpp:523-638),
-    // Russian roulette and scoring.  Must be called by all 32 lanes.  LEAN (the
-    // persistent multi-job kernel, which holds more state per lane) keeps the voxel
-    // read after the truncation test and one interaction pass per event type: the
-    // overlapped reads and the merged pass cost that kernel more spills than they save.
-    template <int MODEL, bool PALETTE, bool LEAN = false, class Real>
-    __device__ __forceinline__ void advance(LaneT<Real>& s, WarpTally& wt, const TransportParams& p, const float* L, const PaletteEntry* pal,
-        bool drain, int interact_t)
+    template <class Real, class Index>
+    __device__ __forceinline__ void take_history(LaneT<Real, Index>& s, const TransportParams& p, uint64_t h)
+    {
+        const bool inside = sample_history(s.ph, s.rng, p, h);
+        s.start_photon();
+        if (!inside)
+            s.state = IDLE;
+    }
+
+    // The ids of one unit of a job's work (see WorkSplit); a unit past the end starts at
+    // or after the job's last id.
+    __device__ __forceinline__ uint64_t work_unit(const WorkSplit& w, uint64_t unit, uint64_t& end)
+    {
+        const bool large = unit < w.large_units;
+        const uint64_t first = large ? unit * w.large : w.large_units * w.large + (unit - w.large_units) * w.small;
+        end = first + (large ? w.large : w.small);
+        return first;
+    }
+
+    // Photons sampled ahead for one warp (shared memory, one row per field).  All 32
+    // lanes sample together, whatever their own photons do; idle lanes then take photons
+    // from here.  Sampling in place, 13 lanes at a time, took 20 % of the instructions
+    // of the CT workload.
+    template <class Real>
+    struct PhotonPool {
+        struct alignas(4 * sizeof(Real)) Quad {
+            Real v[4];
+        };
+        Quad position[32]; // and energy
+        Quad direction[32]; // and weight
+        uint4 rng[32];
+
+        __device__ __forceinline__ void put(int i, const PhotonT<Real>& ph, const Rng& r)
+        {
+            position[i] = Quad { { ph.px, ph.py, ph.pz, ph.energy } };
+            direction[i] = Quad { { ph.dx, ph.dy, ph.dz, ph.weight } };
+            rng[i] = make_uint4(r.s0, r.s1, r.s2, r.s3);
+        }
+        __device__ __forceinline__ void get(int i, PhotonT<Real>& ph, Rng& r) const
+        {
+            const Quad a = position[i], b = direction[i];
+            const uint4 q = rng[i];
+            ph = PhotonT<Real> { a.v[0], a.v[1], a.v[2], b.v[0], b.v[1], b.v[2], a.v[3], b.v[3] };
+            r.s0 = q.x;
+            r.s1 = q.y;
+            r.s2 = q.z;
+            r.s3 = q.w;
+        }
+    };
+
+    // In double precision the three exponentials of the shares cost more than two
+    // registers: the shares of the event types stay with the cached material.
+    template <class Real, bool FAST>
+    constexpr bool keeps_shares = !FAST && sizeof(Real) == 8;
+
+    // attenuation (1 / cm) x stepK (mm) -> event probability
+    template <class Real>
+    constexpr Real per_step = Real(1.0) / (Real(10.0) * Real(0.693147180559945));
+
+    // Photoelectric share, and photoelectric + Compton share, of a material's attenuation.
+    template <class Real>
+    __device__ __forceinline__ void type_shares(const float* L, const LutMeta& m, int mat, Real energy, Real& p0, Real& p01)
+    {
+        const Real logE = m_log10(energy);
+        Real a0, a1, a2;
+        lut_attenuation(L, m, mat, logE, lut_segment(L, m, logE), a0, a1, a2);
+        const Real inv = Real(1.0) / (a0 + a1 + a2);
+        p0 = a0 * inv;
+        p01 = (a0 + a1) * inv;
+    }
+
+    // Russian roulette (transport.hpp:684-694) after an interaction or a forced step.
+    template <class Real, class Index>
+    __device__ __forceinline__ void roulette(LaneT<Real, Index>& s)
+    {
+        if (s.ph.energy * s.ph.weight < Real(ROULETTE_THRESHOLD_D)) {
+            if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D))
+                s.state = IDLE;
+            else
+                s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
+        }
+        s.arm();
+    }
+
+    // The collision test at the end of a flight drawn with the majorant scale 1 / cinv:
+    // a real event (the lane waits for the interaction pass), a virtual collision with
+    // Russian roulette, or the forced scoring of a measurement voxel.
+    template <int MODEL, bool PALETTE, bool FORCED, bool FAST, class Real, class Index>
+    __device__ __forceinline__ void collide(LaneT<Real, Index>& s, WarpState& ws, const TransportParams& p, const float* L, const PaletteEntry* pal,
+        const float* table, const VoxelRaw<PALETTE>& raw, Real cinv)
+    {
+        const LutMeta& m = p.lut_meta;
+        constexpr bool SHARES = keeps_shares<Real, FAST>;
+        Real density;
+        int mat;
+        bool measured;
+        decode_voxel<PALETTE>(raw, pal, density, mat, measured);
+        Real probInv;
+        if constexpr (FAST) {
+            probInv = table[mat * ATT_TABLE_LANES];
+        } else {
+            if (mat != s.cached_mat) {
+                Real a0, a1, a2;
+                lut_attenuation(L, m, mat, s.logE, s.seg, a0, a1, a2);
+                const Real total = a0 + a1 + a2;
+                s.probInv = total * s.stepK * per_step<Real>;
+                s.cached_mat = mat;
+                if constexpr (SHARES) {
+                    const Real inv = Real(1.0) / total;
+                    s.p0 = a0 * inv;
+                    s.p01 = (a0 + a1) * inv;
+                }
+            }
+            probInv = s.probInv;
+        }
+        const Real eventProb = probInv * density * cinv;
+        if (!FORCED || !measured) {
+            // naive sampling (computeInteractions): the event runs in the interaction pass
+            if (static_cast<Real>(s.rng.uniform()) < eventProb) {
+                s.state = 1 + mat;
+            } else if (s.armed) {
+                // virtual collision: Russian roulette (transport.hpp:684-694)
+                if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D)) {
+                    s.state = IDLE;
+                } else {
+                    s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
+                    s.arm();
+                }
+            }
+        } else {
+            // forced photoelectric scoring (computeInteractionsForced): score the forced
+            // photoelectric share now; a real Compton or Rayleigh event goes through the
+            // interaction pass and the weight correction (1 - wc) is applied after it
+            Real photoProb, unused;
+            if constexpr (SHARES)
+                photoProb = s.p0;
+            else
+                type_shares(L, m, mat, s.ph.energy, photoProb, unused);
+            const Real wc = eventProb * photoProb;
+            PhotonT<Real> forced = s.ph;
+            const Real ef = photo_absorption<MODEL>(L, m, forced, mat, s.rng, !FAST && p.normalize_direction);
+            const Real forced_deposit = (forced.energy < Real(ENERGY_CUTOFF_D) ? (ef + forced.energy) : ef) * forced.weight * wc;
+            if (isfinite(forced_deposit)) {
+                score<FAST>(p, s.vidx, forced_deposit);
+                atomicAdd(&ws.forced_deposits, 1u);
+                if (static_cast<Real>(s.rng.uniform()) < eventProb * (Real(1.0) - photoProb)) {
+                    s.forced_wc = wc;
+                    s.state = -1 - mat;
+                } else {
+                    s.ph.weight *= (Real(1.0) - wc);
+                    roulette(s);
+                }
+            } else {
+                atomicAdd(&ws.overflows, 1u);
+                s.state = IDLE;
+            }
+        }
+    }
+
+    // One iteration of the warp-synchronous loop for every lane of the warp: up to
+    // woodcock_burst Woodcock flights for lanes without a pending event
+    // (transport.hpp:650-699), the interaction pass once enough lanes wait
+    // (transport.hpp:523-638), Russian roulette and scoring.  Must be called by all 32
+    // lanes.
+    //
+    // FORCED: the world has a measurement map (forced photoelectric scoring); worlds
+    // without one run a kernel that does not hold that code.  FAST: the job's options are
+    // those of TransportVariant::fast, and `table` (shared memory, one column of lanes per
+    // material) holds the event probability per unit density of every material at the
+    // lane's energy, filled when the energy changes, with most lanes of the warp in step;
+    // otherwise the lane evaluates the material it meets and keeps the last one.  LEAN
+    // (the persistent multi-job kernel,
+    // which holds more state per lane) reads the voxel after the truncation test.
+    template <int MODEL, bool PALETTE, bool FORCED, bool FAST, bool LEAN = false, class Real, class Index>
+    __device__ __forceinline__ void advance(LaneT<Real, Index>& s, WarpState& ws, const TransportParams& p, const float* L, const PaletteEntry* pal,
+        float* table, bool drain, int interact_t)
     {
         const LutMeta& m = p.lut_meta;
         const WorldParams& w = p.world;
-        bool do_score = false;
-        Real deposit = Real(0.0); // energy imparted x weight to score
-        bool check_roulette = false;
+        constexpr bool SHARES = keeps_shares<Real, FAST>;
 
-        if (s.alive && s.pending == EV_NONE) {
-            if (s.updateMax) {
-                s.logE = m_log10(s.ph.energy);
-                s.seg = lut_segment(L, m, s.logE);
-                s.stepK = lut_max_inverse(L, m, s.logE, s.seg) * (Real(10.0) * Real(0.693147180559945)); // cm -> mm, log2 -> ln
-                s.updateMax = false;
-                s.cached_mat = -1;
-                if (p.majorant.cells)
-                    fetch_cell(s, p);
+        // ---- setup -----------------------------------------------------------------------
+        if (s.state == SETUP || s.state == REACH) {
+            if (s.state == SETUP) {
+                const Real logE = m_log10(s.ph.energy);
+                const int seg = lut_segment(L, m, logE);
+                s.stepK = lut_max_inverse(L, m, logE, seg) * (Real(10.0) * Real(0.693147180559945)); // cm -> mm, log2 -> ln
+                if constexpr (FAST) {
+                    for (int mat = 0; mat < m.n_materials; ++mat) {
+                        Real a0, a1, a2;
+                        lut_attenuation(L, m, mat, logE, seg, a0, a1, a2);
+                        table[mat * ATT_TABLE_LANES] = (a0 + a1 + a2) * s.stepK * per_step<Real>;
+                    }
+                } else {
+                    s.logE = logE;
+                    s.seg = seg;
+                    s.cached_mat = -1;
+                }
+                if (FAST || p.majorant.cells)
+                    fetch_cell(s, p, logE);
             }
-            // Up to p.woodcock_burst Woodcock steps per iteration: a lane keeps stepping
-            // through virtual collisions and stops at a real event, the grid boundary or a
-            // forced-scoring voxel.  Each lane draws its own stream in the reference's
-            // order, so the burst length changes the schedule, not the histories.
-            const int burst = max(p.woodcock_burst, 1); // at least one step: every iteration makes progress
-            if (s.hist_steps > MAX_STEPS_PER_HISTORY) {
-                // bounded work per history (checked per burst: at most burst - 1 steps over)
-                atomicAdd(&wt.overflows, 1ull);
-                s.alive = false;
-            }
-            for (int k = 0; k < burst && s.alive; ++k) {
+            // the slab test of the body box runs here, once per iteration for every lane
+            // that needs it: in the flight loop 6 of 18 lanes took it in nearly every
+            // flight, 22 % of the instructions of the CT workload
+            if (s.cR < Real(0.0))
+                s.cR = reach_to_box(s.ph, p.majorant, -s.cR);
+            s.state = FLYING;
+        }
+        if (s.state == FLYING && s.hist_steps > MAX_STEPS_PER_HISTORY) {
+            // bounded work per history (checked per burst: at most burst - 1 steps over)
+            atomicAdd(&ws.overflows, 1u);
+            s.state = IDLE;
+        }
+
+        // ---- flights ---------------------------------------------------------------------
+        // Up to p.woodcock_burst Woodcock steps per iteration, while at least MIN_FLYING
+        // lanes still fly: a lane keeps stepping through virtual collisions and stops at a
+        // real event, the grid boundary or a forced-scoring voxel.  Each lane draws its own
+        // stream in the reference's order, so the burst length changes the schedule, not
+        // the histories.
+        const int burst = max(p.woodcock_burst, 1); // at least one step: every iteration makes progress
+        for (int k = 0; k < burst; ++k) {
+            if (__popc(__ballot_sync(FULL_MASK, s.state == FLYING)) < (k ? MIN_FLYING : 1))
+                break;
+            if (s.state == FLYING) {
                 // a flight drawn with the local majorant ends without a collision test
                 // where that majorant stops holding (truncated: drawn again from there)
-                Real R = s.cR;
-                if (R < Real(0.0))
-                    R = reach_to_box(s.ph, p.majorant, -R);
                 const Real flight = -m_log2(static_cast<Real>(s.rng.uniform_open())) * (s.stepK * s.cinv);
+                const Real R = m_abs(s.cR);
                 const bool truncated = flight > R;
-                const Real step = m_min(flight, R);
-                s.ph.px = m_fma(s.ph.dx, step, s.ph.px);
-                s.ph.py = m_fma(s.ph.dy, step, s.ph.py);
-                s.ph.pz = m_fma(s.ph.dz, step, s.ph.pz);
-                // grid coordinates (p - lo) / spacing as one FMA each, rounded down; the photon
-                // is inside while all three lie in [0, dims) (one unsigned compare each: a
-                // negative or saturated conversion falls outside), which bounds the voxel index
-                const int jx = m_floor_int(m_fma(s.ph.px, w.inv_spacing[0], -w.lo_inv[0]));
-                const int jy = m_floor_int(m_fma(s.ph.py, w.inv_spacing[1], -w.lo_inv[1]));
-                const int jz = m_floor_int(m_fma(s.ph.pz, w.inv_spacing[2], -w.lo_inv[2]));
-                if (!(static_cast<uint32_t>(jx) < w.dims[0] && static_cast<uint32_t>(jy) < w.dims[1]
-                        && static_cast<uint32_t>(jz) < w.dims[2])) {
-                    s.alive = false;
-                    break;
-                }
-                ++s.hist_steps;
-                const uint32_t ix = static_cast<uint32_t>(jx);
-                const uint32_t iy = static_cast<uint32_t>(jy);
-                const uint32_t iz = static_cast<uint32_t>(jz);
-                const Real cinv = s.cinv; // the majorant this flight was drawn with
-                // the voxel is read before the majorant cell, so that the two L2 reads
-                // overlap (a truncated flight does not use the voxel)
-                VoxelRaw<PALETTE> raw {};
-                if constexpr (!LEAN) {
-                    if constexpr (PALETTE) // compact worlds have fewer than 2^32 voxels (world upload)
-                        s.vidx = iz * static_cast<uint32_t>(w.nxy) + (iy * w.dims[0] + ix);
-                    else
-                        s.vidx = static_cast<uint64_t>(iz) * w.nxy + static_cast<uint64_t>(iy) * w.dims[0] + ix;
-                    raw = load_voxel<PALETTE>(w, s.vidx);
-                }
-                if (p.majorant.cells) {
-                    const MajorantGrid& g = p.majorant;
-                    const uint32_t c = (iz >> g.shift[2]) * g.nxy + (iy >> g.shift[1]) * g.nx + (ix >> g.shift[0]);
-                    const float2 cell = __ldg(g.cells + (c * g.bands + s.band));
-                    s.cinv = cell.x;
-                    s.cR = cell.y;
-                }
-                if (truncated)
-                    continue;
-                if constexpr (LEAN) {
-                    if constexpr (PALETTE)
-                        s.vidx = iz * static_cast<uint32_t>(w.nxy) + (iy * w.dims[0] + ix);
-                    else
-                        s.vidx = static_cast<uint64_t>(iz) * w.nxy + static_cast<uint64_t>(iy) * w.dims[0] + ix;
-                    raw = load_voxel<PALETTE>(w, s.vidx);
-                }
-                Real density;
-                int mat;
-                bool measured;
-                decode_voxel<PALETTE>(raw, pal, density, mat, measured);
-                if (mat != s.cached_mat) {
-                    Real a0, a1, a2;
-                    lut_attenuation(L, m, mat, s.logE, s.seg, a0, a1, a2);
-                    const Real attTot = a0 + a1 + a2;
-                    const Real inv = Real(1.0) / attTot;
-                    s.probInv = attTot * s.stepK * (Real(1.0) / (Real(10.0) * Real(0.693147180559945)));
-                    s.p0 = a0 * inv;
-                    s.p01 = (a0 + a1) * inv;
-                    s.cached_mat = mat;
-                }
-                const Real eventProb = s.probInv * density * cinv;
-                if (!measured) {
-                    // naive sampling (computeInteractions): decide the event type now,
-                    // run it in the interaction pass
-                    if (static_cast<Real>(s.rng.uniform()) < eventProb) {
-                        const Real r3 = static_cast<Real>(s.rng.uniform());
-                        s.pending = r3 < s.p0 ? EV_PHOTO : (r3 < s.p01 ? EV_COMPTON : EV_RAYLEIGH);
-                        break;
-                    }
-                    // virtual collision: Russian roulette (transport.hpp:684-694)
-                    if (s.armed) {
-                        if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D)) {
-                            s.alive = false;
-                            break;
-                        }
-                        s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
-                        s.arm();
-                    }
+                if (truncated && s.cR < Real(0.0)) {
+                    // outside the body box the flight may reach further than the ball:
+                    // drawn again once the setup stage has looked how far
+                    s.rng.step_back();
+                    s.state = REACH;
                 } else {
-                    // forced photoelectric scoring (computeInteractionsForced): score the forced
-                    // photoelectric share now; a real Compton or Rayleigh event goes through the
-                    // interaction passes and the weight correction (1 - wc) is applied after it
-                    const Real photoProb = s.p0;
-                    s.forced_wc = eventProb * photoProb;
-                    {
-                        PhotonT<Real> forced = s.ph;
-                        const Real ef = photo_absorption<MODEL>(L, m, forced, mat, s.rng, p.normalize_direction);
-                        deposit = (forced.energy < Real(ENERGY_CUTOFF_D) ? (ef + forced.energy) : ef) * forced.weight * s.forced_wc;
-                        do_score = true;
-                    }
-                    if (static_cast<Real>(s.rng.uniform()) < eventProb * (Real(1.0) - photoProb)) {
-                        s.pending = static_cast<Real>(s.rng.uniform()) * (Real(1.0) - s.p0) < s.p01 - s.p0 ? EV_COMPTON : EV_RAYLEIGH;
+                    const Real step = m_min(flight, R);
+                    s.ph.px = m_fma(s.ph.dx, step, s.ph.px);
+                    s.ph.py = m_fma(s.ph.dy, step, s.ph.py);
+                    s.ph.pz = m_fma(s.ph.dz, step, s.ph.pz);
+                    // grid coordinates (p - lo) / spacing as one FMA each, rounded down; the photon
+                    // is inside while all three lie in [0, dims) (one unsigned compare each: a
+                    // negative or saturated conversion falls outside), which bounds the voxel index
+                    const uint32_t ix = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.px, w.inv_spacing[0], -w.lo_inv[0])));
+                    const uint32_t iy = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.py, w.inv_spacing[1], -w.lo_inv[1])));
+                    const uint32_t iz = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.pz, w.inv_spacing[2], -w.lo_inv[2])));
+                    if (!(ix < w.dims[0] && iy < w.dims[1] && iz < w.dims[2])) {
+                        s.state = IDLE;
                     } else {
-                        s.ph.weight *= (Real(1.0) - s.forced_wc);
-                        s.forced_wc = Real(0.0);
-                        check_roulette = true;
+                        ++s.hist_steps;
+                        const Real cinv = s.cinv; // the majorant this flight was drawn with
+                        // the voxel is read before the majorant cell, so that the two L2 reads
+                        // overlap (a truncated flight does not use the voxel)
+                        VoxelRaw<PALETTE> raw {};
+                        if constexpr (!LEAN) {
+                            s.vidx = voxel_index<PALETTE>(w, ix, iy, iz);
+                            raw = load_voxel<PALETTE>(w, s.vidx);
+                        }
+                        if (FAST || p.majorant.cells) {
+                            const MajorantGrid& g = p.majorant;
+                            const uint32_t c = (iz >> g.shift[2]) * g.nxy + (iy >> g.shift[1]) * g.nx + (ix >> g.shift[0]);
+                            const float2 cell = __ldg(g.cells + (c * g.bands + s.band));
+                            s.cinv = cell.x;
+                            s.cR = cell.y;
+                        }
+                        if (!truncated) {
+                            if constexpr (LEAN) {
+                                s.vidx = voxel_index<PALETTE>(w, ix, iy, iz);
+                                raw = load_voxel<PALETTE>(w, s.vidx);
+                            }
+                            collide<MODEL, PALETTE, FORCED, FAST>(s, ws, p, L, pal, table, raw, cinv);
+                        }
                     }
-                    break; // the forced deposit is scored before the next step
                 }
             }
-        }
-        if (do_score) {
-            // the forced photoelectric deposit is scored before this lane's
-            // interaction pass can add a second deposit in the same iteration
-            if (isfinite(deposit)) {
-                score(p, s.vidx, deposit);
-                atomicAdd(&wt.deposits, 1ull);
-            } else {
-                atomicAdd(&wt.overflows, 1ull);
-                s.alive = false;
-                s.pending = EV_NONE;
-            }
-            do_score = false;
         }
 
-        // ---- interaction passes, one converged pass per event type ---------------------
-        if constexpr (MODEL == 1 && !LEAN) {
-            // LIVERMORE: Compton and Rayleigh both draw one quantile from an energy-row
-            // table and rotate the direction, and photoabsorption only ends the photon,
-            // so every waiting lane runs in one pass (Rayleigh lanes ride along instead
-            // of waiting for a pass of their own).  Each lane draws from its stream in
-            // the order of compton_scatter<1> / rayleigh_scatter<1>.
-            const unsigned waiting = __ballot_sync(FULL_MASK, s.pending != EV_NONE);
-            const unsigned can_step = __ballot_sync(FULL_MASK, s.alive && s.pending == EV_NONE);
-            if (waiting && (__popc(waiting) >= interact_t || can_step == 0u || drain) && s.pending != EV_NONE) {
-                const Real E = s.ph.energy;
-                if (s.pending == EV_PHOTO) {
-                    // photo_absorption<1>: the photon ends and deposits its energy
-                    deposit = E * s.ph.weight;
+        // ---- interaction pass -----------------------------------------------------------
+        // Every waiting lane runs in one pass once enough of them wait.  Photoelectric,
+        // Compton and Rayleigh lanes share the type draw, for LIVERMORE the table quantile
+        // (Compton and Rayleigh angles both come from an energy-row table), the azimuth and
+        // the rotation; each lane draws from its stream in the order of the reference's
+        // samplers.
+        const unsigned waiting = __ballot_sync(FULL_MASK, waits_for_event(s.state));
+        const unsigned can_step = __ballot_sync(FULL_MASK, s.state == FLYING || s.state == REACH);
+        if (!waiting || !(__popc(waiting) >= interact_t || can_step == 0u || drain))
+            return;
+        bool do_score = false;
+        Real deposit = Real(0.0); // energy imparted x weight to score
+        if (waits_for_event(s.state)) {
+            const bool forced = FORCED && s.state < 0;
+            const int mat = (forced ? -s.state : s.state) - 1;
+            s.state = FLYING;
+            const Real E = s.ph.energy;
+            Real p0, p01;
+            if constexpr (SHARES) {
+                p0 = s.p0;
+                p01 = s.p01;
+            } else {
+                type_shares(L, m, mat, E, p0, p01);
+            }
+            const Real r3 = static_cast<Real>(s.rng.uniform());
+            const bool photo = !forced && r3 < p0;
+            const bool compton = forced ? r3 * (Real(1.0) - p0) < p01 - p0 : (!photo && r3 < p01);
+            Real imparted = Real(0.0), cosA = Real(1.0);
+            bool turn = true;
+            bool ok = true; // false: a sampling loop hit its cap
+            if constexpr (MODEL == 1) {
+                if (photo) {
+                    imparted = E;
                     s.ph.energy = Real(0.0);
-                    s.alive = false;
+                    turn = false;
                 } else {
-                    const bool compton = s.pending == EV_COMPTON;
                     Real fe;
                     const int row = table_row(m, E, fe);
-                    const float* tab = p.lut + (compton ? m.off_csf : m.off_ray) + (s.cached_mat * m.tab_ne + row) * (m.tab_nu + 1);
+                    const float* tab = p.lut + (compton ? m.off_csf : m.off_ray) + (mat * m.tab_ne + row) * (m.tab_nu + 1);
                     const Real x = table_quantile(tab, m.tab_nu, static_cast<Real>(s.rng.uniform()), fe);
-                    Real cosA, e = Real(1.0);
                     if (compton) {
-                        // (e - e_min) / (1 - e_min) = x
-                        const Real k = E / Real(ELECTRON_REST_MASS_D);
-                        const Real emin = Real(1.0) / (Real(1.0) + Real(2.0) * k);
-                        const Real one_minus_e = (Real(1.0) - x) * (Real(1.0) - emin);
-                        e = Real(1.0) - one_minus_e;
-                        cosA = m_max(Real(1.0) - one_minus_e / (k * e), -Real(1.0));
+                        Real e;
+                        compton_from_fraction(E, x, e, cosA);
+                        s.ph.energy = E * e;
+                        imparted = E - s.ph.energy;
                     } else {
                         cosA = Real(1.0) - Real(2.0) * x; // q^2 / q_max^2 = (1 - cos) / 2
                     }
-                    const Real phi = rng_azimuth<Real>(s.rng);
-                    peturb(s.ph.dx, s.ph.dy, s.ph.dz, cosA, phi, p.normalize_direction);
-                    if (compton) {
-                        s.ph.energy = E * e;
-                        if (s.ph.energy < Real(ENERGY_CUTOFF_D)) {
-                            deposit = ((E - s.ph.energy) + s.ph.energy) * s.ph.weight;
-                            s.ph.energy = Real(0.0);
-                            s.alive = false;
-                        } else {
-                            deposit = (E - s.ph.energy) * s.ph.weight;
-                            s.updateMax = true;
-                        }
-                    }
                 }
-                do_score = s.pending != EV_RAYLEIGH;
-                if (s.alive && s.forced_wc != Real(0.0))
-                    s.ph.weight *= (Real(1.0) - s.forced_wc);
-                s.forced_wc = Real(0.0);
-                check_roulette = s.alive;
-                s.pending = EV_NONE;
-            }
-        } else {
-            // Rayleigh events are rare (about one in ten interactions here), so their pass
-            // waits until RAYLEIGH_THRESHOLD lanes have one, or until nothing else can run
-            const unsigned ray = __ballot_sync(FULL_MASK, s.pending == EV_RAYLEIGH);
-            const unsigned waiting = __ballot_sync(FULL_MASK, s.pending != EV_NONE);
-            const unsigned can_step = __ballot_sync(FULL_MASK, s.alive && s.pending == EV_NONE);
-            const unsigned waiting_other = waiting & ~ray;
-            const bool stuck = can_step == 0u || drain;
-            const bool run_ray = ray && (__popc(ray) >= RAYLEIGH_THRESHOLD || stuck);
-            if ((waiting_other && (__popc(waiting_other) >= interact_t || stuck)) || run_ray) {
-                const int mat = s.cached_mat;
-                if (__any_sync(FULL_MASK, s.pending == EV_PHOTO) && s.pending == EV_PHOTO) {
-                    const Real e = photo_absorption<MODEL>(L, m, s.ph, mat, s.rng, p.normalize_direction);
-                    do_score = true;
-                    if (s.ph.energy < Real(ENERGY_CUTOFF_D)) {
-                        deposit = (e + s.ph.energy) * s.ph.weight;
-                        s.ph.energy = Real(0.0);
-                        s.alive = false;
-                    } else {
-                        deposit = e * s.ph.weight;
-                        s.updateMax = true;
-                    }
-                }
-                if (__any_sync(FULL_MASK, s.pending == EV_COMPTON) && s.pending == EV_COMPTON) {
-                    Real e = Real(0.0);
-                    if (!compton_scatter<MODEL>(L, p.lut, m, s.ph, mat, s.rng, e, p.normalize_direction)) {
-                        atomicAdd(&wt.overflows, 1ull);
-                        s.alive = false;
-                    } else {
-                        do_score = true;
-                        if (s.ph.energy < Real(ENERGY_CUTOFF_D)) {
-                            deposit = (e + s.ph.energy) * s.ph.weight;
-                            s.ph.energy = Real(0.0);
-                            s.alive = false;
-                        } else {
-                            deposit = e * s.ph.weight;
-                            s.updateMax = true;
-                        }
-                    }
-                }
-                if (run_ray && s.pending == EV_RAYLEIGH) {
-                    if (!rayleigh_scatter<MODEL>(L, p.lut, m, s.ph, mat, s.rng, p.normalize_direction)) {
-                        atomicAdd(&wt.overflows, 1ull);
-                        s.alive = false;
-                    }
-                }
-                if (s.pending != EV_NONE && (s.pending != EV_RAYLEIGH || run_ray)) {
-                    if (s.alive && s.forced_wc != Real(0.0))
-                        s.ph.weight *= (Real(1.0) - s.forced_wc);
-                    s.forced_wc = Real(0.0);
-                    check_roulette = s.alive;
-                    s.pending = EV_NONE;
-                }
-            }
-        }
-        if (check_roulette) {
-            // Russian roulette (transport.hpp:684-694) after an interaction or a forced step
-            if (s.ph.energy * s.ph.weight < Real(ROULETTE_THRESHOLD_D)) {
-                if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D))
-                    s.alive = false;
+            } else {
+                if (photo)
+                    imparted = photo_sample<MODEL>(L, m, s.ph.energy, mat, s.rng, cosA, turn);
+                else if (compton)
+                    ok = compton_sample<MODEL>(L, p.lut, m, s.ph.energy, mat, s.rng, cosA, imparted, turn);
                 else
-                    s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
+                    ok = rayleigh_sample<MODEL>(p.lut, m, E, mat, s.rng, cosA);
             }
-            s.arm();
-        }
-        if (do_score && !isfinite(deposit)) {
-            // never let a non-finite value into the FP64 accumulators: end the
-            // history and report it through the overflow counter
-            do_score = false;
-            s.alive = false;
-            atomicAdd(&wt.overflows, 1ull);
+            if (turn && ok) {
+                const Real phi = rng_azimuth<Real>(s.rng);
+                peturb(s.ph.dx, s.ph.dy, s.ph.dz, cosA, phi, !FAST && p.normalize_direction);
+            }
+            if (!ok) {
+                atomicAdd(&ws.overflows, 1u);
+                s.state = IDLE;
+            } else if (photo || compton) {
+                do_score = true;
+                if (s.ph.energy < Real(ENERGY_CUTOFF_D)) {
+                    deposit = add_rounded(imparted, s.ph.energy) * s.ph.weight;
+                    s.ph.energy = Real(0.0);
+                    s.state = IDLE;
+                } else {
+                    deposit = imparted * s.ph.weight;
+                    s.state = SETUP;
+                }
+            }
+            if (s.state != IDLE) {
+                if (forced)
+                    s.ph.weight *= (Real(1.0) - s.forced_wc);
+                roulette(s);
+            }
+            if (do_score && !isfinite(deposit)) {
+                // never let a non-finite value into the FP64 accumulators: end the
+                // history and report it through the overflow counter
+                do_score = false;
+                s.state = IDLE;
+                atomicAdd(&ws.overflows, 1u);
+            }
         }
         // ---- scoring; the warp is converged here ----------------------------------------
         const unsigned scoring = __ballot_sync(FULL_MASK, do_score);
-        if (p.tally_mode == 2) {
+        if (!FAST && p.tally_mode == 2) {
             if (do_score)
                 score_aggregated(p, scoring, s.vidx, deposit);
         } else if (do_score) {
-            score(p, s.vidx, deposit);
+            score<FAST>(p, s.vidx, deposit);
         }
         if ((threadIdx.x & 31) == 0)
-            wt.deposits += __popc(scoring);
+            ws.deposits += __popc(scoring);
     }
 
     // Counts the steps of the photons a warp's lanes finished (before they are
     // refilled or at a flush).  Called by all 32 lanes.
-    template <class Real>
-    __device__ __forceinline__ void count_steps(LaneT<Real>& s, WarpTally& wt, bool finished)
+    template <class Real, class Index>
+    __device__ __forceinline__ void count_steps(LaneT<Real, Index>& s, WarpState& ws, bool finished)
     {
         const unsigned n = __reduce_add_sync(FULL_MASK, finished ? s.hist_steps : 0u);
         if ((threadIdx.x & 31) == 0)
-            wt.steps += n;
+            ws.steps += n;
         if (finished)
             s.hist_steps = 0;
     }
 
-    // Adds the warp's counters to a job's counters and clears them.  Called by all 32 lanes.
-    template <class Real>
-    __device__ __forceinline__ void flush_counters(LaneT<Real>& s, WarpTally& wt, JobCounters* c)
+    // Adds the warp's counters to a job's counters, the steps of photons in flight
+    // included, and clears them.  Called by all 32 lanes.
+    template <class Real, class Index>
+    __device__ __forceinline__ void flush_counters(LaneT<Real, Index>& s, WarpState& ws, JobCounters* c)
     {
-        count_steps(s, wt, true); // counted once: the photons' steps so far
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) {
-            if (wt.steps)
-                atomicAdd(&c->steps, wt.steps);
-            if (wt.deposits)
-                atomicAdd(&c->deposits, wt.deposits);
-            if (wt.overflows)
-                atomicAdd(&c->overflows, wt.overflows);
-            if (wt.histories)
-                atomicAdd(&c->histories_done, wt.histories);
-            wt = WarpTally {};
-        }
-        __syncwarp();
+        count_steps(s, ws, true); // counted once: the photons' steps so far
+        add_counters(ws, c);
     }
 
     // ---- single-job transport kernel ----------------------------------------------------
     //
-    // Warp-synchronous loop.  Each iteration every lane with a live photon and no
-    // pending interaction takes up to woodcock_burst Woodcock steps; a real event
-    // only records its type (photoelectric / Compton / Rayleigh) and ends the lane's
-    // burst.  The interactions are then run in
-    // one converged pass per type once enough lanes wait, and finished lanes are
-    // refilled together once enough are idle, so the expensive branches run with
-    // many lanes active instead of one or two.
-    // the FP64-everywhere instantiation needs about twice the registers: two blocks per SM
-    template <class Real, int MODEL, bool PALETTE>
-    __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
+    // Warp-synchronous loop, bound by instruction issue at about half of a warp's lanes:
+    // what a stage costs is paid by the warp whatever its lanes, so each stage runs when
+    // enough lanes want it.  Idle lanes take photons from the warp's pool, which all 32
+    // lanes fill together; new photons and new energies are set up together; the lanes
+    // then fly a burst; and once enough of them wait for an event the interactions run in
+    // one pass.  64 registers (four blocks of 256 threads per SM; 48 or 40 registers
+    // spilled and ran 20 to 30 % slower); what belongs to the warp lives in shared memory.
+    // Sampling in place and the box test in the flight loop before; now, kernel alone:
+    // CT 512 x 512 x 200 of 1e8 histories 13.4 -> 12.7 ms, DX 160^3 of 5e6 0.753 -> 0.609 ms,
+    // CTDI phantom of 1e7 with forced scoring 1.29 -> 1.12 ms, DX 96^3 of 1e6 in FP64
+    // 6.4 -> 4.5 ms (two blocks per SM: about twice the registers).
+    template <class Real, int MODEL, bool PALETTE, bool FORCED, bool FAST>
+    __global__ void __launch_bounds__(TRANSPORT_THREADS, sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
     {
         extern __shared__ float4 smem_f4[];
-        const float* L = p.lut;
+        // in the fast kernels a shared-memory address to the compiler (32-bit loads)
+        const float* L = FAST ? reinterpret_cast<const float*>(smem_f4) : p.lut;
         size_t smem_off = 0;
-        if (p.lut_in_smem) {
+        if (FAST || p.lut_in_smem) {
             float4* dst = smem_f4;
             const float4* src = reinterpret_cast<const float4*>(p.lut);
-            const int n4 = (p.lut_meta.total_floats + 3) / 4;
+            const int n4 = ((MODEL == 2 ? p.lut_meta.total_floats : p.lut_meta.off_shells) + 3) / 4;
             for (int i = threadIdx.x; i < n4; i += blockDim.x)
                 dst[i] = __ldg(src + i);
-            L = reinterpret_cast<const float*>(smem_f4);
+            if constexpr (!FAST)
+                L = reinterpret_cast<const float*>(smem_f4);
             smem_off = static_cast<size_t>(n4);
         }
         const PaletteEntry* pal = nullptr;
@@ -1008,69 +1146,107 @@ namespace {
             for (int i = threadIdx.x; i < PALETTE_MAX; i += blockDim.x)
                 spal[i] = i < p.world.palette_n ? p.world.palette[i] : PaletteEntry { Real(0.0), 0u };
             pal = spal;
+            smem_off += PALETTE_MAX * sizeof(PaletteEntry) / sizeof(float4);
         }
+        float* table = nullptr; // this lane's column of the attenuation table
+        if constexpr (FAST)
+            table = reinterpret_cast<float*>(smem_f4 + smem_off) + threadIdx.x;
         __syncthreads();
         const int lane = threadIdx.x & 31;
         const unsigned lanemask_lt = (1u << lane) - 1u;
         const int regen_t = p.regen_threshold;
         const int interact_t = p.interact_threshold;
-        const bool use_queue = p.queue.pos_energy != nullptr;
-        const unsigned long long source_total = use_queue ? p.counters->queue_count : p.total_histories;
-        unsigned long long* source_head = use_queue ? &p.counters->next_photon : &p.counters->next_history;
+        const bool use_queue = !FAST && p.queue.pos_energy != nullptr;
+        const uint64_t source_total = use_queue ? p.counters->queue_count : p.total_histories;
 
-        __shared__ WarpTally tallies[1024 / 32];
-        WarpTally& wt = tallies[threadIdx.x >> 5];
-        if (lane == 0)
-            wt = WarpTally {};
+        __shared__ WarpState states[TRANSPORT_THREADS / 32];
+        __shared__ PhotonPool<Real> pools[TRANSPORT_THREADS / 32];
+        WarpState& ws = states[threadIdx.x >> 5];
+        PhotonPool<Real>& pool = pools[threadIdx.x >> 5];
+        if (lane == 0) {
+            ws = WarpState {};
+            const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+            ws.next = work_unit(p.work, unit, ws.end);
+        }
         __syncwarp();
-        LaneT<Real> s {};
-        s.alive = false;
-        // warp-uniform pool of ids (queue slots or history ids) [pool_next, pool_end)
-        uint64_t pool_next = 0, pool_end = 0;
-        bool exhausted = false;
+        LaneT<Real, typename VoxelRaw<PALETTE>::Index> s {};
+        s.state = IDLE;
+        bool exhausted = false; // no photon left to take
 
         while (true) {
             // ---- refill idle lanes together ------------------------------------------------
-            unsigned need = __ballot_sync(FULL_MASK, !s.alive && !exhausted);
-            const unsigned live = __ballot_sync(FULL_MASK, s.alive);
-            if (need && (__popc(need) >= regen_t || live == 0u)) {
-                while (need && !exhausted) {
-                    if (pool_next >= pool_end) {
-                        unsigned long long base = 0;
-                        if (lane == 0) {
-                            const bool cancelled = p.cancel && *p.cancel;
-                            base = cancelled ? source_total : atomicAdd(source_head, (unsigned long long)WARP_POOL_CHUNK);
+            unsigned need = __ballot_sync(FULL_MASK, s.state == IDLE);
+            if (!exhausted && __popc(need) >= regen_t) {
+                while (need) {
+                    const int pooled = ws.pooled;
+                    if (pooled == 0) {
+                        uint64_t next = ws.next;
+                        if (next >= ws.end) {
+                            // a unit of the job is done: the job's progress, and the next unit
+                            if (ws.histories >= 256)
+                                add_counters(ws, p.counters);
+                            if (lane == 0) {
+                                const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
+                                unsigned long long* head = use_queue ? &p.counters->next_photon : &p.counters->next_history;
+                                const uint64_t unit = warps + atomicAdd(head, 1ull);
+                                uint64_t end;
+                                next = work_unit(p.work, unit, end);
+                                ws.end = end;
+                                // the host's flag costs a read over the link: not at every small unit
+                                if (unit < p.work.large_units && p.cancel && *p.cancel)
+                                    next = source_total;
+                            }
+                            next = __shfl_sync(FULL_MASK, next, 0);
                         }
-                        base = __shfl_sync(FULL_MASK, base, 0);
-                        if (base >= source_total) {
+                        if (next >= source_total) {
                             exhausted = true;
                             break;
                         }
-                        pool_next = base;
-                        pool_end = min(static_cast<uint64_t>(base + WARP_POOL_CHUNK), static_cast<uint64_t>(source_total));
+                        // all lanes sample the next 32 ids; those inside the grid go into the pool
+                        const bool mine = next + lane < source_total;
+                        bool inside = false;
+                        PhotonT<Real> ph {};
+                        Rng rng {};
+                        if (mine) {
+                            if (use_queue) {
+                                load_queued(ph, rng, p.queue, next + lane);
+                                inside = true;
+                            } else {
+                                inside = sample_history(ph, rng, p, next + lane);
+                            }
+                        }
+                        const unsigned sampled = __ballot_sync(FULL_MASK, mine);
+                        const unsigned entered = __ballot_sync(FULL_MASK, inside);
+                        if (inside)
+                            pool.put(__popc(entered & lanemask_lt), ph, rng);
+                        if (lane == 0) {
+                            ws.next = next + 32;
+                            ws.pooled = __popc(entered);
+                            if (!use_queue)
+                                ws.histories += __popc(sampled);
+                        }
+                        __syncwarp();
+                        continue;
                     }
-                    const uint64_t avail = pool_end - pool_next;
-                    const unsigned rank = __popc(need & lanemask_lt);
-                    const bool mine = ((need >> lane) & 1u) && rank < avail;
+                    const int rank = __popc(need & lanemask_lt);
+                    const bool mine = ((need >> lane) & 1u) && rank < pooled;
                     const unsigned taken = __ballot_sync(FULL_MASK, mine);
-                    count_steps(s, wt, mine);
-                    if (lane == 0 && !use_queue)
-                        wt.histories += __popc(taken);
+                    count_steps(s, ws, mine);
                     if (mine) {
-                        if (use_queue) {
-                            take_queued(s, p.queue, pool_next + rank);
-                        } else
-                            take_history(s, p, pool_next + rank);
+                        pool.get(pooled - 1 - rank, s.ph, s.rng);
+                        s.start_photon();
                     }
-                    pool_next += __popc(taken);
+                    if (lane == 0)
+                        ws.pooled = pooled - __popc(taken);
                     need &= ~taken;
+                    __syncwarp(); // the pool may be filled again
                 }
             }
-            if (exhausted && __ballot_sync(FULL_MASK, s.alive) == 0u)
+            if (exhausted && __ballot_sync(FULL_MASK, s.state != IDLE) == 0u)
                 break;
-            advance<MODEL, PALETTE>(s, wt, p, L, pal, exhausted, interact_t);
+            advance<MODEL, PALETTE, FORCED, FAST>(s, ws, p, L, pal, table, exhausted, interact_t);
         }
-        flush_counters(s, wt, p.counters);
+        flush_counters(s, ws, p.counters);
     }
 
     // ---- batched transport kernel ------------------------------------------------------
@@ -1101,13 +1277,13 @@ namespace {
         const int regen_t = ctl->regen_threshold;
         const int interact_t = ctl->interact_threshold;
 
-        __shared__ WarpTally tallies[BATCH_WARPS];
-        WarpTally& wt = tallies[warp];
+        __shared__ WarpState states[BATCH_WARPS];
+        WarpState& ws = states[warp];
         if (lane == 0)
-            wt = WarpTally {};
+            ws = WarpState {};
         __syncwarp();
-        LaneT<float> s {};
-        s.alive = false;
+        LaneT<float, uint64_t> s {};
+        s.state = IDLE;
         int job = -1;
         uint64_t pool_next = 0, pool_end = 0;
         BatchItem next {};
@@ -1115,9 +1291,8 @@ namespace {
         bool exhausted = false;
 
         while (true) {
-            unsigned need = __ballot_sync(FULL_MASK, !s.alive && !exhausted);
-            const unsigned live = __ballot_sync(FULL_MASK, s.alive);
-            if (need && (__popc(need) >= regen_t || live == 0u)) {
+            unsigned need = __ballot_sync(FULL_MASK, s.state == IDLE && !exhausted);
+            if (need && __popc(need) >= regen_t) {
                 while (need && !exhausted) {
                     if (pool_next >= pool_end) {
                         if (!have_next) {
@@ -1134,10 +1309,10 @@ namespace {
                         }
                         if (static_cast<int>(next.job) != job) {
                             // switch jobs only when every lane is idle
-                            if (__ballot_sync(FULL_MASK, s.alive) != 0u)
+                            if (__ballot_sync(FULL_MASK, s.state != IDLE) != 0u)
                                 break;
                             if (job >= 0)
-                                flush_counters(s, wt, p.counters);
+                                flush_counters(s, ws, p.counters);
                             job = static_cast<int>(next.job);
                             __syncwarp();
                             const int* src = reinterpret_cast<const int*>(b.jobs + job);
@@ -1158,27 +1333,27 @@ namespace {
                     const unsigned rank = __popc(need & lanemask_lt);
                     const bool mine = ((need >> lane) & 1u) && rank < avail;
                     const unsigned taken = __ballot_sync(FULL_MASK, mine);
-                    count_steps(s, wt, mine);
+                    count_steps(s, ws, mine);
                     if (lane == 0)
-                        wt.histories += __popc(taken);
+                        ws.histories += __popc(taken);
                     if (mine)
                         take_history(s, p, pool_next + rank);
                     pool_next += __popc(taken);
                     need &= ~taken;
                 }
             }
-            const unsigned live2 = __ballot_sync(FULL_MASK, s.alive);
+            const unsigned live2 = __ballot_sync(FULL_MASK, s.state != IDLE);
             if (exhausted && live2 == 0u)
                 break;
             if (live2 == 0u)
                 continue; // waiting to switch jobs with nothing in flight: refill again
             if (p.world.palette_index)
-                advance<MODEL, true, true>(s, wt, p, p.lut, pal, exhausted || have_next, interact_t);
+                advance<MODEL, true, true, false, true>(s, ws, p, p.lut, pal, nullptr, exhausted || have_next, interact_t);
             else
-                advance<MODEL, false, true>(s, wt, p, p.lut, pal, exhausted || have_next, interact_t);
+                advance<MODEL, false, true, false, true>(s, ws, p, p.lut, pal, nullptr, exhausted || have_next, interact_t);
         }
         if (job >= 0)
-            flush_counters(s, wt, p.counters);
+            flush_counters(s, ws, p.counters);
     }
 
     // ---- photon generation pass ---------------------------------------------------------
@@ -1195,17 +1370,7 @@ namespace {
             PhotonT<float> ph {};
             Rng rng;
             if (i < count) {
-                const uint64_t h = first + i;
-                rng.init(p.seed, h);
-                uint32_t ei;
-                if (p.uniform_hpe && p.total_histories <= 0xffffffffull)
-                    ei = udiv_apply(static_cast<uint32_t>(h), p.hpe_magic, p.hpe_shifts);
-                else
-                    ei = p.uniform_hpe ? static_cast<uint32_t>(h / p.uniform_hpe) : find_exposure(p.source, h);
-                DevExposure ex;
-                load_exposure(p.source.exposures + ei, ex);
-                sample_particle(p.source, ex, rng, ph);
-                inworld = transport_to_world(p.world, ph);
+                inworld = sample_history(ph, rng, p, first + i);
                 ++generated;
             }
             const unsigned mask = __ballot_sync(FULL_MASK, inworld);
@@ -1341,12 +1506,18 @@ namespace {
             PhotonT<float> ph { 0, 0, 0, 0, 0, 1, energy, 1 };
             float dep = 0.0f;
             bool ok = true;
+            float cosA = 1.0f;
+            bool turn = true;
             if (kind == 0)
-                dep = photo_absorption<MODEL>(L, m, ph, material, rng);
+                dep = photo_sample<MODEL>(L, m, ph.energy, material, rng, cosA, turn);
             else if (kind == 1)
-                ok = compton_scatter<MODEL>(L, L, m, ph, material, rng, dep);
+                ok = compton_sample<MODEL>(L, L, m, ph.energy, material, rng, cosA, dep, turn);
             else
-                ok = rayleigh_scatter<MODEL>(L, L, m, ph, material, rng);
+                ok = rayleigh_sample<MODEL>(L, m, ph.energy, material, rng, cosA);
+            if (turn && ok) {
+                const float phi = rng_azimuth<float>(rng);
+                peturb(ph.dx, ph.dy, ph.dz, cosA, phi);
+            }
             const float len = sqrtf(ph.dx * ph.dx + ph.dy * ph.dy + ph.dz * ph.dz);
             out_cos[i] = ok ? (len > 0 ? ph.dz / len : 1.0f) : 2.0f;
             out_energy[i] = ph.energy;
@@ -1392,21 +1563,46 @@ namespace {
 
 } // namespace
 
+// The kernel of a job: one for the options of nearly every job (TransportVariant::fast),
+// without the forced-scoring code where the world has no measurement map, and one for
+// all others.
 template <class Real, int MODEL, bool PALETTE>
-static void* transport_entry() { return reinterpret_cast<void*>(&transport_kernel<Real, MODEL, PALETTE>); }
-
-template <class Real>
-static void* transport_function_as(int model, bool palette)
+static void* transport_entry(bool forced, bool fast)
 {
-    if (palette)
-        return model == 0 ? transport_entry<Real, 0, true>() : (model == 1 ? transport_entry<Real, 1, true>() : transport_entry<Real, 2, true>());
-    return model == 0 ? transport_entry<Real, 0, false>() : (model == 1 ? transport_entry<Real, 1, false>() : transport_entry<Real, 2, false>());
+    if constexpr (sizeof(Real) == 4) {
+        if (fast)
+            return forced ? reinterpret_cast<void*>(&transport_kernel<Real, MODEL, PALETTE, true, true>)
+                          : reinterpret_cast<void*>(&transport_kernel<Real, MODEL, PALETTE, false, true>);
+    }
+    return reinterpret_cast<void*>(&transport_kernel<Real, MODEL, PALETTE, true, false>);
 }
 
-// precision 0: FP32 transport (the fast path); 1: FP64 everywhere (the precision study)
-static void* transport_function(int model, bool palette, int precision)
+template <class Real>
+static void* transport_function_as(int model, bool palette, bool forced, bool fast)
 {
-    return precision == 1 ? transport_function_as<double>(model, palette) : transport_function_as<float>(model, palette);
+    if (palette)
+        return model == 0 ? transport_entry<Real, 0, true>(forced, fast)
+                          : (model == 1 ? transport_entry<Real, 1, true>(forced, fast) : transport_entry<Real, 2, true>(forced, fast));
+    return model == 0 ? transport_entry<Real, 0, false>(forced, fast)
+                      : (model == 1 ? transport_entry<Real, 1, false>(forced, fast) : transport_entry<Real, 2, false>(forced, fast));
+}
+
+static void* transport_function(const TransportVariant& v)
+{
+    return v.precision == 1 ? transport_function_as<double>(v.model, v.palette, true, false)
+                            : transport_function_as<float>(v.model, v.palette, v.forced, v.fast);
+}
+
+TransportVariant transport_variant(const TransportParams& p, int model, bool queued)
+{
+    TransportVariant v;
+    v.model = model;
+    v.precision = p.precision;
+    v.palette = p.world.palette_index != nullptr;
+    v.forced = p.world.has_measurement != 0;
+    v.fast = p.precision != 1 && p.lut_meta.n_materials <= ATT_TABLE_MATERIALS && p.lut_in_smem && p.majorant.cells && p.records && p.tally_mode == 0
+        && !p.normalize_direction && !queued;
+    return v;
 }
 
 const void* batch_kernel_function(int model)
@@ -1437,46 +1633,69 @@ cudaError_t launch_generate(const TransportParams& p, uint64_t first, uint64_t c
     return cudaGetLastError();
 }
 
-size_t transport_smem_bytes(size_t lut_bytes, bool lut_in_smem, bool palette)
+size_t transport_smem_bytes(const TransportVariant& v, const LutMeta& meta, bool lut_in_smem)
 {
-    size_t b = lut_in_smem ? (lut_bytes + 15) / 16 * 16 : 0;
-    if (palette)
+    size_t b = lut_in_smem ? (static_cast<size_t>(staged_lut_floats(meta, v.model)) * sizeof(float) + 15) / 16 * 16 : 0;
+    if (v.palette)
         b += PALETTE_MAX * sizeof(PaletteEntry);
+    if (v.fast)
+        b += static_cast<size_t>(meta.n_materials) * ATT_TABLE_LANES * sizeof(float);
     return b;
+}
+
+WorkSplit transport_work_split(uint64_t histories, uint64_t warps, bool queued)
+{
+    WorkSplit w;
+    if (queued || warps == 0) { // how many photons wait is known on the device only
+        w.large_units = ~0ull >> 16;
+        return w;
+    }
+    const uint64_t rounds = (histories + warps * 32 - 1) / (warps * 32);
+    if (rounds <= 2) {
+        w.large_units = 0;
+    } else if (rounds <= 24) {
+        w.large = static_cast<uint32_t>(rounds * 3 / 4) * 32;
+        w.large_units = std::min(warps, histories / w.large);
+    } else {
+        const uint64_t tail = warps * 32 * 6;
+        w.large_units = (histories - tail) / w.large;
+        w.small = 64;
+    }
+    return w;
 }
 
 cudaError_t launch_transport(const TransportParams& p, int model, int grid, int block, size_t smem, cudaStream_t stream)
 {
-    const bool palette = p.world.palette_index != nullptr;
-    void* fn = transport_function(model, palette, p.precision);
+    void* fn = transport_function(transport_variant(p, model, p.queue.pos_energy != nullptr));
     void* args[] = { const_cast<TransportParams*>(&p) };
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, stream);
 }
 
 cudaError_t preload_transport_kernels()
 {
-    for (int precision = 0; precision < 2; ++precision)
-        for (int model = 0; model < 3; ++model)
-            for (int palette = 0; palette < 2; ++palette) {
+    for (int model = 0; model < 3; ++model)
+        for (int palette = 0; palette < 2; ++palette)
+            for (int kind = 0; kind < 4; ++kind) { // FP64; FP32 general, fast, fast with forced scoring
+                const TransportVariant v { model, kind == 0 ? 1 : 0, palette != 0, kind != 2, kind >= 2 };
                 cudaFuncAttributes attr {};
-                const cudaError_t e = cudaFuncGetAttributes(&attr, transport_function(model, palette != 0, precision));
+                const cudaError_t e = cudaFuncGetAttributes(&attr, transport_function(v));
                 if (e != cudaSuccess)
                     return e;
             }
     return cudaSuccess;
 }
 
-int transport_max_blocks_per_sm(int model, bool palette, int block, size_t smem, int precision)
+int transport_max_blocks_per_sm(const TransportVariant& v, int block, size_t smem)
 {
-    void* fn = transport_function(model, palette, precision);
+    void* fn = transport_function(v);
     // The dynamic shared-memory limit is a property of the function, read when a
     // launch (or a graph holding it) is made: it only ever grows, so launches
     // queued or captured earlier with larger LUTs stay valid.
     static std::mutex m;
-    static int limit[12] = {};
+    static std::unordered_map<void*, int> limit;
     {
         std::lock_guard<std::mutex> lock(m);
-        int& cur = limit[(precision == 1 ? 6 : 0) + model * 2 + (palette ? 1 : 0)];
+        int& cur = limit[fn];
         if (static_cast<int>(smem) > cur) {
             if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess)
                 cur = static_cast<int>(smem);
