@@ -1256,6 +1256,8 @@ try {
     off = align_up(off + static_cast<size_t>(R) * 2, 4);
     m.off_shells = static_cast<int>(off);
     off = align_up(off + static_cast<size_t>(nm) * dev::N_SHELLS * dev::SHELL_FLOATS, 4);
+    m.off_shell_sums = static_cast<int>(off);
+    off = align_up(off + static_cast<size_t>(nm) * dev::SHELL_SUM_FLOATS, 4);
     m.total_floats = static_cast<int>(off);
     std::vector<float> img(off, 0.0f);
     for (int i = 0; i < R; ++i)
@@ -1277,6 +1279,12 @@ try {
                 o[5 + k] = static_cast<float>(c.line_probabilities[k]);
                 o[8 + k] = static_cast<float>(c.line_energies[k]);
             }
+            // the partial sums, in the order and precision of the kernels'
+            float* sums = img.data() + m.off_shell_sums + mat * dev::SHELL_SUM_FLOATS;
+            const float electrons = o[2] > 0.0f ? o[1] : 0.0f;
+            sums[s] = s > 0 ? sums[s - 1] + electrons : electrons;
+            sums[dev::N_SHELLS + s] = s > 0 ? sums[dev::N_SHELLS + s - 1] + o[3] : o[3];
+            sums[2 * dev::N_SHELLS] = s > 0 ? std::max(sums[2 * dev::N_SHELLS], o[0]) : o[0];
         }
     }
     // inverse-CDF sampling tables for the Compton and Rayleigh samplers, after the

@@ -52,6 +52,7 @@ struct LutMeta {
     int off_coef;    // n_materials * R * 6
     int off_maxcoef; // R * 2
     int off_shells;  // n_materials * 12 * SHELL_FLOATS (read by the impulse-approximation model only)
+    int off_shell_sums; // n_materials * SHELL_SUM_FLOATS (as the shells)
     // inverse-CDF sampling tables, after total_floats (read from global memory,
     // not staged in shared memory): rows of tab_nu + 1 quantiles
     int off_ckn;     // Compton energy fraction, no scatter factor: tab_ne rows
@@ -60,7 +61,6 @@ struct LutMeta {
     int tab_ne, tab_nu;
     float tab_le0;     // ln of the first table energy
     float tab_inv_dle; // 1 / ln step
-    int pad0;
 };
 
 __device__ __forceinline__ float exp10_fast(float y) { return exp2f(y * 3.32192809488736f); }
@@ -137,6 +137,7 @@ __device__ __forceinline__ Real table_quantile(const float* row, int nu, Real u,
 
 constexpr int SHELL_FLOATS = 12; // binding, nElectrons, J0, photoProb, yield, lineP[3], lineE[3], pad
 constexpr int N_SHELLS = 12;
+constexpr int SHELL_SUM_FLOATS = 28; // partial sums over the shells: electrons (J0 > 0)[12], photoProb[12], highest binding energy, pad
 
 constexpr float KEV_TO_ANGSTROM = 12.398520f;
 constexpr float ELECTRON_REST_MASS = 510.9989461f;
