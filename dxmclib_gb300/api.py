@@ -1572,9 +1572,8 @@ class Job:
         if out is not None:
             dose, var, nev = out
         else:
-            dose = np.zeros(n)
-            var = np.zeros(n)
-            nev = np.zeros(n, np.uint32) if want_events else None
+            dose, var = np.empty(n), np.empty(n)
+            nev = np.empty(n, np.uint32) if want_events else None
         st = A.JobStats()
         rc = self.ctx.lib.dxmc_gpu_job_result(self.handle, output_mode, calibration, dose.ctypes.data_as(A.DP),
                                               var.ctypes.data_as(A.DP),
@@ -1583,6 +1582,10 @@ class Job:
                      rejection_overflows=st.rejection_overflows, kernel_ms=st.kernel_ms, job_ms=st.job_ms, status=rc)
         if check and rc not in (A.DXMC_OK,):
             A.check(rc, self.ctx.handle, "dxmc_gpu_job_result")
+        if out is None and rc not in (A.DXMC_OK, A.DXMC_ERR_REJECTION_CAP, A.DXMC_ERR_CANCELLED):
+            for a in (dose, var, nev):  # nothing was written
+                if a is not None:
+                    a.fill(0)
         return dose, var, nev, stats
 
     def result_async(self, output_mode: int = A.OUTPUT_EV_PER_HISTORY, calibration: float = 1.0, out=None,
@@ -1782,14 +1785,15 @@ class Transport:
         return self._ctx
 
     def __call__(self, world: World, source: Source, progressbar=None, useSourceDoseCalibration: bool = True) -> Result:
-        n = world.size()
-        empty = Result(np.zeros(n), np.zeros(n, np.uint32), np.zeros(n))
+        def empty():
+            n = world.size()
+            return Result(np.zeros(n), np.zeros(n, np.uint32), np.zeros(n))
         if not world.isValid() or source is None:
-            return empty
+            return empty()
         source.updateFromWorld(world)
         source.validate()
         if not source.isValid():
-            return empty
+            return empty()
         beams = source.beams(world.directionCosines())
         histories = int(sum(int(np.sum(b.exposures.n_histories)) for b in beams))
         dworld = DeviceWorld(self._ctx, world)

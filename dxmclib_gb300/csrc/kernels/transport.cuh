@@ -219,17 +219,18 @@ int transport_max_blocks_per_sm(const TransportVariant& v, int block, size_t sme
 size_t transport_smem_bytes(const TransportVariant& v, const LutMeta& meta, bool lut_in_smem);
 // Post-processing of the tallies into dose / variance (densities from the world's layout).
 // dose, variance and counts_out may be device memory or page-locked host memory
-// (written through its device mapping); counts_out, if not null, gets a copy of counts.
+// (written through its device mapping); counts_out, if not null, gets a copy of counts,
+// counters_out one of the job's counters.
 cudaError_t launch_postprocess(const double* tally, const WorldParams& w, uint64_t n,
     int mode, double histories, double voxel_volume_cm3, double calibration, double* dose, double* variance,
     const uint32_t* counts, uint32_t* counts_out, cudaStream_t stream);
 cudaError_t launch_postprocess_records(const TallyRecord* records, const WorldParams& w, uint64_t n,
     int mode, double histories, double voxel_volume_cm3, double calibration, double* dose, double* variance,
-    uint32_t* counts_out, cudaStream_t stream);
+    uint32_t* counts_out, const JobCounters* counters, JobCounters* counters_out, cudaStream_t stream);
 // The same with float results (Result<float>: 12 bytes per voxel with the counts).
 cudaError_t launch_postprocess_records_f32(const TallyRecord* records, const WorldParams& w, uint64_t n,
     int mode, double histories, double voxel_volume_cm3, double calibration, float* dose, float* variance,
-    uint32_t* counts_out, cudaStream_t stream);
+    uint32_t* counts_out, const JobCounters* counters, JobCounters* counters_out, cudaStream_t stream);
 cudaError_t launch_postprocess_f32(const float* tally, const WorldParams& w, uint64_t n,
     int mode, double histories, double voxel_volume_cm3, double calibration, double* dose, double* variance,
     const uint32_t* counts, uint32_t* counts_out, cudaStream_t stream);

@@ -1534,8 +1534,10 @@ namespace {
     __global__ void postprocess_records_kernel(const TallyRecord* __restrict__ rec, const Voxel* __restrict__ voxels,
         const uint8_t* __restrict__ palette_index, const PaletteEntry* __restrict__ palette, uint64_t n, int mode,
         double histories, double voxel_volume_cm3, double calibration, OutT* __restrict__ dose, OutT* __restrict__ variance,
-        uint32_t* __restrict__ counts_out)
+        uint32_t* __restrict__ counts_out, const JobCounters* counters, JobCounters* counters_out)
     {
+        if (counters_out && blockIdx.x == 0 && threadIdx.x == 0)
+            *counters_out = *counters; // the job has ended; saves a copy of its own
         const double h_inv = 1.0 / (histories - 1.0);
         const double h_d = 1.0e3 / histories;
         const double h_v = 1.0e6 / histories;
@@ -1822,23 +1824,23 @@ cudaError_t launch_postprocess(const double* tally, const WorldParams& w, uint64
 
 cudaError_t launch_postprocess_records(const TallyRecord* records, const WorldParams& w, uint64_t n, int mode,
     double histories, double voxel_volume_cm3, double calibration, double* dose, double* variance, uint32_t* counts_out,
-    cudaStream_t stream)
+    const JobCounters* counters, JobCounters* counters_out, cudaStream_t stream)
 {
     const int block = 256;
     const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 152ull * 16));
     postprocess_records_kernel<double><<<grid, block, 0, stream>>>(records, w.palette_index ? nullptr : w.voxels, w.palette_index,
-        w.palette, n, mode, histories, voxel_volume_cm3, calibration, dose, variance, counts_out);
+        w.palette, n, mode, histories, voxel_volume_cm3, calibration, dose, variance, counts_out, counters, counters_out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_postprocess_records_f32(const TallyRecord* records, const WorldParams& w, uint64_t n, int mode,
     double histories, double voxel_volume_cm3, double calibration, float* dose, float* variance, uint32_t* counts_out,
-    cudaStream_t stream)
+    const JobCounters* counters, JobCounters* counters_out, cudaStream_t stream)
 {
     const int block = 256;
     const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 152ull * 16));
     postprocess_records_kernel<float><<<grid, block, 0, stream>>>(records, w.palette_index ? nullptr : w.voxels, w.palette_index,
-        w.palette, n, mode, histories, voxel_volume_cm3, calibration, dose, variance, counts_out);
+        w.palette, n, mode, histories, voxel_volume_cm3, calibration, dose, variance, counts_out, counters, counters_out);
     return cudaGetLastError();
 }
 
