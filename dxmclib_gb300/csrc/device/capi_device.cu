@@ -40,7 +40,7 @@ constexpr int DEFAULT_WOODCOCK_BURST = DXMC_DEFAULT_WOODCOCK_BURST; // Woodcock 
 // With local majorants a history takes fewer, more varied steps: shorter bursts
 // and a later refill keep more lanes of a warp stepping together.
 constexpr int DEFAULT_LOCAL_REGEN_THRESHOLD = 4;
-constexpr int DEFAULT_LOCAL_WOODCOCK_BURST = 3;
+constexpr int DEFAULT_LOCAL_WOODCOCK_BURST = 0; // by the stops per flight a warp has seen
 // Local-majorant grid: target cell edge and energy bands (above 15 keV)
 #ifndef DXMC_MAJORANT_CELL_MM
 #define DXMC_MAJORANT_CELL_MM 6.0
