@@ -961,6 +961,9 @@ namespace {
                 const Real logE = m_log10(s.ph.energy);
                 const int seg = lut_segment(L, m, logE);
                 s.stepK = lut_max_inverse(L, m, logE, seg) * (Real(10.0) * Real(0.693147180559945)); // cm -> mm, log2 -> ln
+                // the cell is read before the attenuations, whose arithmetic hides its latency
+                if (FAST || p.majorant.cells)
+                    fetch_cell(s, p, logE);
                 if constexpr (FAST) {
                     for (int mat = 0; mat < m.n_materials; ++mat) {
                         Real a0, a1, a2;
@@ -972,8 +975,6 @@ namespace {
                     s.seg = seg;
                     s.cached_mat = -1;
                 }
-                if (FAST || p.majorant.cells)
-                    fetch_cell(s, p, logE);
             }
             // the slab test of the body box runs here, once per iteration for every lane
             // that needs it: in the flight loop 6 of 18 lanes took it in nearly every
@@ -1055,8 +1056,9 @@ namespace {
         // the rotation; each lane draws from its stream in the order of the reference's
         // samplers.
         const unsigned waiting = __ballot_sync(FULL_MASK, waits_for_event(s.state));
-        const unsigned can_step = __ballot_sync(FULL_MASK, s.state == FLYING || s.state == REACH);
-        if (!waiting || !(__popc(waiting) >= interact_t || can_step == 0u || drain))
+        if (!waiting)
+            return;
+        if (__popc(waiting) < interact_t && !drain && __any_sync(FULL_MASK, s.state == FLYING || s.state == REACH))
             return;
         bool do_score = false;
         Real deposit = Real(0.0); // energy imparted x weight to score
@@ -1190,15 +1192,15 @@ namespace {
             }
         }
         // ---- scoring; the warp is converged here ----------------------------------------
-        const unsigned scoring = __ballot_sync(FULL_MASK, do_score);
         if (!FAST && p.tally_mode == 2) {
+            const unsigned scoring = __ballot_sync(FULL_MASK, do_score);
             if (do_score)
                 score_aggregated(p, scoring, s.vidx, deposit);
         } else if (do_score) {
             score<FAST>(p, s.vidx, deposit);
         }
-        if ((threadIdx.x & 31) == 0)
-            ws.deposits += __popc(scoring);
+        if (do_score)
+            atomicAdd(&ws.deposits, 1u);
     }
 
     // Counts the steps of the photons a warp's lanes finished (before they are
