@@ -205,6 +205,7 @@ struct dxmc_gpu_ctx {
     static constexpr int ASYNC_STREAMS = 4;
     cudaStream_t async_streams[ASYNC_STREAMS] {};
     int next_async = 0;
+    cudaStream_t piece_stream = nullptr; // every other piece of a large result
     // world and table uploads: their copies and host waits do not queue behind
     // the jobs on the context stream (uploading the next world overlaps a job)
     cudaStream_t upload_stream = nullptr;
@@ -846,7 +847,8 @@ try {
     int least_priority = 0, greatest_priority = 0;
     cudaDeviceGetStreamPriorityRange(&least_priority, &greatest_priority);
     const int result_priority = std::min(least_priority, greatest_priority + 1);
-    bool streams = cudaStreamCreateWithPriority(&ctx->result_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess;
+    bool streams = cudaStreamCreateWithPriority(&ctx->result_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess
+        && cudaStreamCreateWithPriority(&ctx->piece_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess;
     for (cudaStream_t& r : ctx->async_streams)
         streams = streams && cudaStreamCreateWithPriority(&r, cudaStreamNonBlocking, result_priority) == cudaSuccess;
     streams = streams && cudaStreamCreateWithPriority(&ctx->upload_stream, cudaStreamNonBlocking, greatest_priority) == cudaSuccess;
@@ -2004,7 +2006,7 @@ LaunchPlan plan_launch(dxmc_gpu_ctx* ctx, const dxmc_lut* lut, const dxmc_job_de
     const dev::TransportVariant variant = dev::transport_variant(p, model, queued);
     L.smem = dev::transport_smem_bytes(variant, lut->meta, p.lut_in_smem != 0);
     L.block = jd->block_size == 128 || jd->block_size == 256 ? jd->block_size
-                                                              : (ctx->options.block_size > 0 ? ctx->options.block_size : dev::TRANSPORT_THREADS);
+                                                              : (ctx->options.block_size > 0 ? ctx->options.block_size : dev::transport_block(variant.fast, variant.forced, variant.palette, model));
     // also sets the kernel's dynamic shared-memory limit for this launch
     const int occ = dev::transport_max_blocks_per_sm(variant, L.block, L.smem);
     int per_sm = jd->blocks_per_sm > 0 ? std::min(jd->blocks_per_sm, std::max(occ, 1))
@@ -2600,7 +2602,7 @@ void wait_unused(dxmc_gpu_ctx* ctx, const Usage& u)
 
 void destroy_ctx_streams(dxmc_gpu_ctx* ctx)
 {
-    for (cudaStream_t st : { ctx->stream, ctx->result_stream, ctx->upload_stream })
+    for (cudaStream_t st : { ctx->stream, ctx->result_stream, ctx->piece_stream, ctx->upload_stream })
         if (st)
             cudaStreamDestroy(st);
     for (cudaStream_t st : ctx->async_streams)
@@ -2612,6 +2614,7 @@ void sync_ctx_streams(dxmc_gpu_ctx* ctx)
 {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->result_stream);
+    cudaStreamSynchronize(ctx->piece_stream);
     for (cudaStream_t r : ctx->async_streams)
         if (r)
             cudaStreamSynchronize(r);
@@ -3021,7 +3024,7 @@ try {
         const uint64_t pieces = nv * per_voxel > PIECED_RESULT_BYTES ? 8 : 1;
         cudaStream_t streams[2] = { s, s };
         if (pieces > 1) {
-            streams[1] = ctx->async_streams[ctx->next_async];
+            streams[1] = ctx->piece_stream;
             if (e == cudaSuccess)
                 e = cudaEventCreateWithFlags(&other_done, cudaEventDisableTiming);
             if (e == cudaSuccess)

@@ -401,7 +401,7 @@ try {
         p.lut_in_smem = lut_bytes <= smem_limit ? 1 : 0;
         const dev::TransportVariant variant = dev::transport_variant(p, jd->model, false);
         const size_t smem = dev::transport_smem_bytes(variant, meta, p.lut_in_smem != 0);
-        const int block = dev::TRANSPORT_THREADS;
+        const int block = dev::transport_block(variant.fast, variant.forced, variant.palette, jd->model);
         int per_sm = dev::transport_max_blocks_per_sm(variant, block, smem);
         if (per_sm <= 0)
             per_sm = 1;

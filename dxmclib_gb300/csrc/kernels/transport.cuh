@@ -198,7 +198,16 @@ struct TransportVariant {
 // in 1 KB per warp; filling a column costs about 20 instructions per material
 // when a photon's energy changes, which beyond eight exceeds what it saves.
 constexpr int ATT_TABLE_MATERIALS = 8;
-constexpr int TRANSPORT_THREADS = 256; // largest block of the single-job kernels
+constexpr int TRANSPORT_THREADS = 288; // largest block of the single-job kernels
+// Default block of a variant, four of which fill an SM's registers (two in FP64).  Where
+// 56 registers a thread are enough, nine warps a block: the 36 warps of an SM hide more of
+// the reads' latency than 32 with 64 registers (CT 512 x 512 x 100 of 2e7 histories 2.32 ->
+// 2.26 ms; the forced-scoring, impulse-approximation and 8-byte-voxel kernels spill and lose
+// 7, 8 and 1 %).
+__host__ __device__ constexpr int transport_block(bool fast, bool forced, bool palette, int model)
+{
+    return fast && !forced && palette && model != 2 ? TRANSPORT_THREADS : 256;
+}
 // The part of the LUT image a kernel stages in shared memory.
 inline int staged_lut_floats(const LutMeta& m, int model) { return model == 2 ? m.total_floats : m.off_shells; }
 constexpr int ATT_TABLE_LANES = TRANSPORT_THREADS;

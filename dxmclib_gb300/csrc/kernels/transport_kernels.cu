@@ -593,7 +593,7 @@ namespace {
     }
 
 #ifndef DXMC_MIN_BLOCKS_PER_SM
-#define DXMC_MIN_BLOCKS_PER_SM 4 // resident 256-thread blocks per SM the register budget must allow (64 registers)
+#define DXMC_MIN_BLOCKS_PER_SM 4 // resident blocks per SM the register budget must allow (64 or 56 registers, see transport_block)
 #endif
 
     // Flights per iteration of the loop.  A lane that stops waits for the end of the burst,
@@ -1238,7 +1238,7 @@ namespace {
     // CTDI phantom of 1e7 with forced scoring 1.29 -> 1.12 ms, DX 96^3 of 1e6 in FP64
     // 6.4 -> 4.5 ms (two blocks per SM: about twice the registers).
     template <class Real, int MODEL, bool PALETTE, bool FORCED, bool FAST>
-    __global__ void __launch_bounds__(TRANSPORT_THREADS, sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
+    __global__ void __launch_bounds__(transport_block(FAST, FORCED, PALETTE, MODEL), sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
     {
         extern __shared__ float4 smem_f4[];
         // in the fast kernels a shared-memory address to the compiler (32-bit loads)
@@ -1273,8 +1273,9 @@ namespace {
         const bool use_queue = !FAST && p.queue.pos_energy != nullptr;
         const uint64_t source_total = use_queue ? p.counters->queue_count : p.total_histories;
 
-        __shared__ WarpState states[TRANSPORT_THREADS / 32];
-        __shared__ PhotonPool<Real> pools[TRANSPORT_THREADS / 32];
+        constexpr int WARPS = transport_block(FAST, FORCED, PALETTE, MODEL) / 32;
+        __shared__ WarpState states[WARPS];
+        __shared__ PhotonPool<Real> pools[WARPS];
         WarpState& ws = states[threadIdx.x >> 5];
         PhotonPool<Real>& pool = pools[threadIdx.x >> 5];
         if (lane == 0) {
