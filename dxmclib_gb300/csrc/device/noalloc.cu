@@ -381,6 +381,7 @@ try {
         p.tally = tally;
         p.tally_f32 = nullptr;
         p.n_events = n_events;
+        p.tally_copies = 1;
         p.counters = reinterpret_cast<dev::JobCounters*>(s + OFF_COUNTERS);
         p.cancel = nullptr;
         p.total_histories = total;

@@ -46,12 +46,18 @@ namespace {
 #endif
     }
 
+    // The copy of the records that this block adds to.
+    __device__ __forceinline__ TallyRecord* tally_records(const TransportParams& p)
+    {
+        return p.records + (blockIdx.x & (p.tally_copies - 1)) * p.world.n_voxels;
+    }
+
     template <bool FAST, class Real>
     __device__ __forceinline__ void score(const TransportParams& p, uint64_t idx, Real e)
     {
         if (FAST || p.records) {
             const double ed = static_cast<double>(e);
-            score_record(p.records + idx, ed, ed * ed, 1u);
+            score_record(tally_records(p) + idx, ed, ed * ed, 1u);
             return;
         }
         if constexpr (FAST)
@@ -90,7 +96,7 @@ namespace {
         }
         if (lane == leader) {
             if (p.records) {
-                score_record(p.records + idx, static_cast<double>(sum), static_cast<double>(sum2), count);
+                score_record(tally_records(p) + idx, static_cast<double>(sum), static_cast<double>(sum2), count);
             } else {
                 double* t = p.tally + 2 * idx;
                 atomicAdd(t, static_cast<double>(sum));
@@ -1549,6 +1555,26 @@ namespace {
         }
     }
 
+    // Copies 1 .. copies - 1 of the records added to copy 0, in that order.
+    __global__ void fold_tallies_kernel(TallyRecord* __restrict__ rec, uint64_t n, uint32_t copies)
+    {
+        for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+            uint32_t events = 0;
+            double e = 0.0, ee = 0.0;
+            for (uint32_t c = 1; c < copies; ++c) {
+                const TallyRecord r = rec[c * n + i];
+                events += r.events;
+                e += r.energy;
+                ee += r.energy2;
+            }
+            if (events) {
+                rec[i].energy += e;
+                rec[i].energy2 += ee;
+                rec[i].events += events;
+            }
+        }
+    }
+
     // Post-processing from tally records: one 32-byte record read per voxel; the
     // results in double (Result<double>) or float (Result<float>), computed in double.
     template <typename OutT>
@@ -1840,6 +1866,14 @@ cudaError_t launch_postprocess(const double* tally, const WorldParams& w, uint64
     const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 152ull * 16));
     postprocess_kernel<double><<<grid, block, 0, stream>>>(tally, w.palette_index ? nullptr : w.voxels, w.palette_index, w.palette, n, mode,
         histories, voxel_volume_cm3, calibration, dose, variance, counts, counts_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fold_tallies(TallyRecord* records, uint64_t n, uint32_t copies, cudaStream_t stream)
+{
+    const int block = 256;
+    const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 152ull * 8));
+    fold_tallies_kernel<<<grid, block, 0, stream>>>(records, n, copies);
     return cudaGetLastError();
 }
 

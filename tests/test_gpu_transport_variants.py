@@ -85,3 +85,30 @@ def test_work_split_takes_every_history_once(gpu_ctx, histories):
     _same(usual, _run(gpu_ctx, dworld, dlut, src, 1, {"queue_log2_chunk": 19}))
     dlut.close()
     dworld.close()
+
+
+@pytest.mark.parametrize("model", [1, 2])
+@pytest.mark.parametrize("histories", [499_990, 500_000, 700_010])
+def test_pencil_tally_copies(gpu_ctx, model, histories):
+    """A pencil beam's job of 5e5 histories or more adds to copies of the tally; a member
+    of a persistent batch has one.  A finished job's preview is its raw energy tally."""
+    import dxmclib_gb300 as dx
+    from dxmclib_gb300 import _capi as A
+    w = _world(2, False, np.random.default_rng(3))
+    dworld = dx.DeviceWorld(gpu_ctx, w)
+    dlut = dx.DeviceLut(gpu_ctx, dx.LutBlob(w.materialMap(), dworld.max_density(), 150.0))
+    src = dx.PencilSource()
+    src.setPosition((0.0, 0.0, -200.0))
+    src.setDirectionCosines((1, 0, 0, 0, 1, 0))
+    src.setPhotonEnergy(60.0)
+    src.setTotalExposures(10)
+    src.setHistoriesPerExposure(histories // 10)
+    job = dx.Job(gpu_ctx, dworld, dlut, src.exposures(), seed=11, model=model)
+    alone = job.result(A.OUTPUT_RAW)
+    np.testing.assert_array_equal(job.preview(), alone[0])
+    job.close()
+    batch = dx.Batch(gpu_ctx, [dx.BatchEntry(dworld, dlut, src.exposures(), seed=11, model=model)], mode=dx.Batch.PERSISTENT)
+    _same(alone, batch.jobs[0].result(A.OUTPUT_RAW))
+    batch.close()
+    dlut.close()
+    dworld.close()
