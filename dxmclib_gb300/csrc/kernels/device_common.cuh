@@ -100,14 +100,31 @@ __device__ __forceinline__ double m_floor(double a) { return floor(a); }
 __device__ __forceinline__ int m_floor_int(float a) { return __float2int_rd(a); }
 __device__ __forceinline__ int m_floor_int(double a) { return __double2int_rd(a); }
 
-// Rows of the sampling tables around energy E: row i and i + 1 with weight f of
+// A stored float in the precision a kernel computes in.  To double by integer
+// operations: the FP64 kernels used to convert the same table and grid constants at every
+// use, 226 conversions per history, and 56 are left (DX 96^3 of 1e6 histories 4.57 ->
+// 4.41 ms; the FP64 pipe, 86 % busy at one warp instruction per 16 cycles and SM, bounds them).
+template <class Real>
+__device__ __forceinline__ Real up(float x);
+template <>
+__device__ __forceinline__ float up<float>(float x) { return x; }
+template <>
+__device__ __forceinline__ double up<double>(float x)
+{
+    const uint32_t u = __float_as_uint(x), magnitude = u & 0x7fffffffu;
+    if (magnitude - 0x00800000u >= 0x7f000000u) // zero, subnormal, infinity, NaN
+        return static_cast<double>(x);
+    return __hiloint2double(static_cast<int>((u & 0x80000000u) | ((magnitude >> 3) + 0x38000000u)), static_cast<int>(u << 29));
+}
+
+// Rows of the sampling tables around energy E (lnE: its logarithm): row i and i + 1 with weight f of
 // the upper one.  Draws interpolate the two rows' quantiles at the same level
 // (quantile interpolation), which follows distributions that stretch with
 // energy far more closely than a mixture of the rows would.
 template <class Real>
-__device__ __forceinline__ int table_row(const LutMeta& m, Real E, Real& f)
+__device__ __forceinline__ int table_row(const LutMeta& m, Real lnE, Real& f)
 {
-    const Real t = (m_log(E) - m.tab_le0) * m.tab_inv_dle;
+    const Real t = (lnE - up<Real>(m.tab_le0)) * up<Real>(m.tab_inv_dle);
     int i = static_cast<int>(m_floor(t));
     f = t - static_cast<Real>(i);
     if (i < 0) {
@@ -128,8 +145,8 @@ __device__ __forceinline__ Real table_quantile(const float* row, int nu, Real u,
     const Real pos = u * static_cast<Real>(nu);
     const int j = min(static_cast<int>(pos), nu - 1);
     const Real f = pos - static_cast<Real>(j);
-    const Real a0 = __ldg(row + j), b0 = __ldg(row + j + 1);
-    const Real a1 = __ldg(row + nu + 1 + j), b1 = __ldg(row + nu + 1 + j + 1);
+    const Real a0 = up<Real>(__ldg(row + j)), b0 = up<Real>(__ldg(row + j + 1));
+    const Real a1 = up<Real>(__ldg(row + nu + 1 + j)), b1 = up<Real>(__ldg(row + nu + 1 + j + 1));
     const Real q0 = m_fma(f, b0 - a0, a0);
     const Real q1 = m_fma(f, b1 - a1, a1);
     return m_fma(fe, q1 - q0, q0);
@@ -212,11 +229,12 @@ struct Rng {
     __device__ __forceinline__ float azimuth() { return fmaf(uniform(), 6.28318530717959f, -3.14159265358979f); }
 };
 
-// azimuth uniform in [-pi, pi) in the kernel's precision, from the same 23-bit draw
-template <class Real>
-__device__ __forceinline__ Real rng_azimuth(Rng& r)
+// Sine and cosine of an azimuth uniform in [-pi, pi) in the kernel's precision, from the
+// same 23-bit draw (in double of pi times 2 u - 1, which is exact).
+__device__ __forceinline__ void rng_azimuth(Rng& r, float* s, float* c) { m_sincos(r.azimuth(), s, c); }
+__device__ __forceinline__ void rng_azimuth(Rng& r, double* s, double* c)
 {
-    return m_fma(static_cast<Real>(r.uniform()), Real(2.0 * PI_D), Real(-PI_D));
+    sincospi(fma(up<double>(r.uniform()), 2.0, -1.0), s, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -224,12 +242,10 @@ __device__ __forceinline__ Real rng_azimuth(Rng& r)
 // ---------------------------------------------------------------------------
 
 // vectormath::rotate (vectormath.hpp:83-99): Rodrigues rotation about a (not
-// necessarily unit) axis.
+// necessarily unit) axis, by an angle of sine s and cosine c.
 template <class Real>
-__device__ __forceinline__ void rotate(Real& vx, Real& vy, Real& vz, Real ax, Real ay, Real az, Real angle)
+__device__ __forceinline__ void rotate(Real& vx, Real& vy, Real& vz, Real ax, Real ay, Real az, Real s, Real c)
 {
-    Real s, c;
-    m_sincos(angle, &s, &c);
     const Real midt = (Real(1) - c) * (vx * ax + vy * ay + vz * az);
     const Real ox = c * vx + midt * ax + s * (ay * vz - az * vy);
     const Real oy = c * vy + midt * ay + s * (-ax * vz + az * vx);
@@ -239,15 +255,23 @@ __device__ __forceinline__ void rotate(Real& vx, Real& vy, Real& vz, Real ax, Re
     vz = oz;
 }
 
+template <class Real>
+__device__ __forceinline__ void rotate(Real& vx, Real& vy, Real& vz, Real ax, Real ay, Real az, Real angle)
+{
+    Real s, c;
+    m_sincos(angle, &s, &c);
+    rotate(vx, vy, vz, ax, ay, az, s, c);
+}
+
 // vectormath::peturb (vectormath.hpp:197-221), including its quirk: the
 // orthogonal axis cross(vec, e_k) is never normalised, so |dir| shrinks after
 // every direction change exactly as in the reference (and the angle between the
 // old and new direction is not theta).  normalize = true scales the axis to unit
 // length first: a unit direction then turns by exactly theta and stays a unit
 // vector (the normalised physics mode; it does not match the reference).  Takes
-// cos(theta).
+// cos(theta) and the sine and cosine of the azimuth.
 template <class Real>
-__device__ __forceinline__ void peturb(Real& vx, Real& vy, Real& vz, Real cos_theta, Real phi, bool normalize = false)
+__device__ __forceinline__ void peturb(Real& vx, Real& vy, Real& vz, Real cos_theta, Real sin_phi, Real cos_phi, bool normalize = false)
 {
     const Real ax = m_abs(vx), ay = m_abs(vy), az = m_abs(vz);
     const int k = ax <= ay ? (ax <= az ? 0 : 2) : (ay <= az ? 1 : 2);
@@ -272,7 +296,7 @@ __device__ __forceinline__ void peturb(Real& vx, Real& vy, Real& vz, Real cos_th
         uy *= inv;
         uz *= inv;
     }
-    rotate(ux, uy, uz, vx, vy, vz, phi);
+    rotate(ux, uy, uz, vx, vy, vz, sin_phi, cos_phi);
     const Real st = m_sqrt(m_max(Real(0), Real(1) - cos_theta * cos_theta));
     vx = vx * cos_theta + ux * st;
     vy = vy * cos_theta + uy * st;
@@ -302,8 +326,8 @@ __device__ __forceinline__ int upper_bound_f(const float* x, int n, Real v)
 template <class Real>
 __device__ __forceinline__ int lut_segment(const float* L, const LutMeta& m, Real logE)
 {
-    if (logE > m.linear_energy) {
-        const int idx = static_cast<int>((logE - m.linear_energy) * m.inv_linear_step) + m.linear_index;
+    if (logE > up<Real>(m.linear_energy)) {
+        const int idx = static_cast<int>((logE - up<Real>(m.linear_energy)) * up<Real>(m.inv_linear_step)) + m.linear_index;
         return min(idx, m.R - 1);
     }
     const int pos = upper_bound_f(L + m.off_x, m.R, logE);
@@ -315,16 +339,16 @@ __device__ __forceinline__ void lut_attenuation(const float* L, const LutMeta& m
 {
     const float2* c = reinterpret_cast<const float2*>(L + m.off_coef + (material * m.R + seg) * 6);
     const float2 p = c[0], q = c[1], r = c[2];
-    photo = m_exp10(m_fma(Real(p.y), logE, Real(p.x)));
-    compt = m_exp10(m_fma(Real(q.y), logE, Real(q.x)));
-    rayl = m_exp10(m_fma(Real(r.y), logE, Real(r.x)));
+    photo = m_exp10(m_fma(up<Real>(p.y), logE, up<Real>(p.x)));
+    compt = m_exp10(m_fma(up<Real>(q.y), logE, up<Real>(q.x)));
+    rayl = m_exp10(m_fma(up<Real>(r.y), logE, up<Real>(r.x)));
 }
 
 template <class Real>
 __device__ __forceinline__ Real lut_max_inverse(const float* L, const LutMeta& m, Real logE, int seg)
 {
     const float2 c = reinterpret_cast<const float2*>(L + m.off_maxcoef)[seg];
-    return m_exp10(m_fma(Real(c.y), logE, Real(c.x)));
+    return m_exp10(m_fma(up<Real>(c.y), logE, up<Real>(c.x)));
 }
 
 } // namespace dxmc_gb300::dev

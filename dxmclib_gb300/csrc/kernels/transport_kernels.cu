@@ -172,20 +172,20 @@ namespace {
             const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
             Real cum[N_SHELLS] = {};
             shell_sums<1>(L, m, E, material, cum);
-            const float* sh = shells + pick_shell(cum, static_cast<Real>(rng.uniform())) * SHELL_FLOATS;
+            const float* sh = shells + pick_shell(cum, up<Real>(rng.uniform())) * SHELL_FLOATS;
             const Real binding = sh[0];
             if (binding > E || binding < Real(ENERGY_CUTOFF_D))
                 return E;
-            const Real r1 = static_cast<Real>(rng.uniform());
+            const Real r1 = up<Real>(rng.uniform());
             if (r1 <= sh[4]) {
                 int line = 0;
-                Real r3 = static_cast<Real>(rng.uniform()) - sh[5];
+                Real r3 = up<Real>(rng.uniform()) - sh[5];
                 while (r3 > Real(0.0) && line < 2) {
                     ++line;
                     r3 -= sh[5 + line];
                 }
                 energy = sh[8 + line];
-                const Real theta = static_cast<Real>(rng.uniform()) * Real(PI_D);
+                const Real theta = up<Real>(rng.uniform()) * Real(PI_D);
                 cosA = m_cos(theta);
                 turn = true;
                 return E - energy;
@@ -202,8 +202,9 @@ namespace {
         bool turn;
         const Real imparted = photo_sample<MODEL>(L, m, ph.energy, material, rng, cosA, turn);
         if (turn) {
-            const Real phi = rng_azimuth<Real>(rng);
-            peturb(ph.dx, ph.dy, ph.dz, cosA, phi, norm);
+            Real sin_phi, cos_phi;
+            rng_azimuth(rng, &sin_phi, &cos_phi);
+            peturb(ph.dx, ph.dy, ph.dz, cosA, sin_phi, cos_phi, norm);
         }
         return imparted;
     }
@@ -215,8 +216,8 @@ namespace {
         if constexpr (MODEL == 0) {
             constexpr Real extreme = Real(1.08866210790363); // 4 sqrt(2) / (3 sqrt(3))
             for (int it = 0; it < REJECTION_CAP; ++it) {
-                const Real r1 = static_cast<Real>(rng.uniform()) * extreme;
-                const Real theta = static_cast<Real>(rng.uniform()) * Real(PI_D);
+                const Real r1 = up<Real>(rng.uniform()) * extreme;
+                const Real theta = up<Real>(rng.uniform()) * Real(PI_D);
                 Real s, c;
                 m_sincos(theta, &s, &c);
                 if (!(r1 > (Real(2.0) - s * s) * s)) {
@@ -229,8 +230,8 @@ namespace {
             // the density of the reference's RITA draw of q^2 <= q_max^2 followed by the
             // (1 + cos^2) / 2 rejection, drawn by inverse CDF: no loop, no divergence
             Real fe;
-            const int row = table_row(m, energy, fe);
-            const Real y = table_quantile(G + m.off_ray + (material * m.tab_ne + row) * (m.tab_nu + 1), m.tab_nu, static_cast<Real>(rng.uniform()), fe);
+            const int row = table_row(m, m_log(energy), fe);
+            const Real y = table_quantile(G + m.off_ray + (material * m.tab_ne + row) * (m.tab_nu + 1), m.tab_nu, up<Real>(rng.uniform()), fe);
             cosA = Real(1.0) - Real(2.0) * y; // q^2 / q_max^2 = (1 - cos) / 2
             return true;
         }
@@ -245,7 +246,7 @@ namespace {
         const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
         Real cum[N_SHELLS] = {};
         shell_sums<0>(L, m, energy, material, cum);
-        const int shell = pick_shell(cum, static_cast<Real>(rng.uniform()));
+        const int shell = pick_shell(cum, up<Real>(rng.uniform()));
         if (!(cum[N_SHELLS - 1] > Real(0.0)))
             return -1;
         const Real U = shells[shell * SHELL_FLOATS] / Real(ELECTRON_REST_MASS_D);
@@ -265,7 +266,7 @@ namespace {
         const Real k = energy / Real(ELECTRON_REST_MASS_D);
         const Real emin = Real(1.0) / (Real(1.0) + Real(2.0) * k);
         const Real gmax_inv = Real(1.0) / (Real(1.0) / emin + emin);
-        const Real r1 = static_cast<Real>(rng.uniform());
+        const Real r1 = up<Real>(rng.uniform());
         // e = r1 + (1 - r1) emin, with 1 - e = (1 - r1)(1 - emin) formed directly so
         // that t stays positive when e rounds to 1 in single precision
         const Real one_minus_e = (Real(1.0) - r1) * (Real(1.0) - emin);
@@ -273,7 +274,7 @@ namespace {
         t = one_minus_e / (k * e);
         const Real sin2 = mul_rounded(t, (Real(2.0) - t));
         const Real g = add_rounded(Real(1.0) / e + e, -sin2) * gmax_inv;
-        const Real r2 = static_cast<Real>(rng.uniform());
+        const Real r2 = up<Real>(rng.uniform());
         return !(r2 > g);
     }
 
@@ -317,7 +318,7 @@ namespace {
         } else {
             S = Real(1.0) - (Real(1.0) - alpha * pU) * expb * Real(0.5);
         }
-        const Real r3 = static_cast<Real>(rng.uniform());
+        const Real r3 = up<Real>(rng.uniform());
         if (r3 > S)
             return false;
         Real Fmax;
@@ -327,7 +328,7 @@ namespace {
             Fmax = Real(1.0) + alpha * pU;
         else
             Fmax = Real(1.0) + alpha * pi;
-        const Real r4 = static_cast<Real>(rng.uniform_open()); // log(rbar2) below needs rbar2 > 0
+        const Real r4 = up<Real>(rng.uniform_open()); // log(rbar2) below needs rbar2 > 0
         const Real rbar2 = Real(2.0) * r4 * expb;
         Real pz;
         if (rbar2 < Real(1.0)) {
@@ -344,7 +345,7 @@ namespace {
             Fpz = Real(1.0) + alpha * pU;
         else
             Fpz = Real(1.0) + alpha * pz;
-        const Real r5 = static_cast<Real>(rng.uniform());
+        const Real r5 = up<Real>(rng.uniform());
         if (r5 > Fpz / Fmax)
             return false;
         const Real part = m_sqrt(m_max(Real(1.0) - Real(2.0) * e * cosA + e * e * (Real(1.0) - pz * pz * sin2), Real(0.0)));
@@ -399,10 +400,10 @@ namespace {
             // the density of the reference's Klein-Nishina rejection (times the scatter
             // factor S(q) for LIVERMORE), drawn by inverse CDF: no loop, no divergence
             Real fe;
-            const int row = table_row(m, E, fe);
+            const int row = table_row(m, m_log(E), fe);
             const float* tab = MODEL == 1 ? G + m.off_csf + (material * m.tab_ne + row) * (m.tab_nu + 1)
                                           : G + m.off_ckn + row * (m.tab_nu + 1);
-            const Real x = table_quantile(tab, m.tab_nu, static_cast<Real>(rng.uniform()), fe);
+            const Real x = table_quantile(tab, m.tab_nu, up<Real>(rng.uniform()), fe);
             compton_from_fraction(E, x, e, cosA);
         }
         energy = E * e;
@@ -414,30 +415,30 @@ namespace {
     template <class Real>
     __device__ __forceinline__ void sample_particle(const SourceParams& s, const DevExposure& ex, Rng& rng, PhotonT<Real>& ph)
     {
-        const Real theta = ex.coll[0] + static_cast<Real>(rng.uniform()) * (ex.coll[1] - ex.coll[0]);
-        const Real phi = ex.coll[2] + static_cast<Real>(rng.uniform()) * (ex.coll[3] - ex.coll[2]);
-        ph.px = ex.pos[0];
-        ph.py = ex.pos[1];
-        ph.pz = ex.pos[2];
-        ph.dx = ex.beam[0];
-        ph.dy = ex.beam[1];
-        ph.dz = ex.beam[2];
-        ph.weight = ex.weight;
-        rotate(ph.dx, ph.dy, ph.dz, Real(ex.cosy[0]), Real(ex.cosy[1]), Real(ex.cosy[2]), theta);
-        rotate(ph.dx, ph.dy, ph.dz, Real(ex.cosx[0]), Real(ex.cosx[1]), Real(ex.cosx[2]), phi);
+        const Real theta = up<Real>(ex.coll[0]) + up<Real>(rng.uniform()) * up<Real>(ex.coll[1] - ex.coll[0]);
+        const Real phi = up<Real>(ex.coll[2]) + up<Real>(rng.uniform()) * up<Real>(ex.coll[3] - ex.coll[2]);
+        ph.px = up<Real>(ex.pos[0]);
+        ph.py = up<Real>(ex.pos[1]);
+        ph.pz = up<Real>(ex.pos[2]);
+        ph.dx = up<Real>(ex.beam[0]);
+        ph.dy = up<Real>(ex.beam[1]);
+        ph.dz = up<Real>(ex.beam[2]);
+        ph.weight = up<Real>(ex.weight);
+        rotate(ph.dx, ph.dy, ph.dz, up<Real>(ex.cosy[0]), up<Real>(ex.cosy[1]), up<Real>(ex.cosy[2]), theta);
+        rotate(ph.dx, ph.dy, ph.dz, up<Real>(ex.cosx[0]), up<Real>(ex.cosx[1]), up<Real>(ex.cosx[2]), phi);
         if (s.spec_n > 0) {
             // SpecterDistribution::sampleValue (dxmcrandom.hpp:322-326)
-            const Real r = static_cast<Real>(rng.uniform());
+            const Real r = up<Real>(rng.uniform());
             const uint32_t k = rng.below(static_cast<uint32_t>(s.spec_n));
-            const uint32_t idx = r < __ldg(s.spec_prob + k) ? k : __ldg(s.spec_alias + k);
+            const uint32_t idx = r < up<Real>(__ldg(s.spec_prob + k)) ? k : __ldg(s.spec_alias + k);
             if (idx + 1 < static_cast<uint32_t>(s.spec_n)) {
-                const Real e0 = __ldg(s.spec_energy + idx), e1 = __ldg(s.spec_energy + idx + 1);
-                ph.energy = e0 + static_cast<Real>(rng.uniform()) * (e1 - e0);
+                const Real e0 = up<Real>(__ldg(s.spec_energy + idx)), e1 = up<Real>(__ldg(s.spec_energy + idx + 1));
+                ph.energy = e0 + up<Real>(rng.uniform()) * (e1 - e0);
             } else {
-                ph.energy = __ldg(s.spec_energy + idx);
+                ph.energy = up<Real>(__ldg(s.spec_energy + idx));
             }
         } else {
-            ph.energy = ex.mono_energy;
+            ph.energy = up<Real>(ex.mono_energy);
         }
         if (s.bowtie_angle) {
             // BowTieFilter::sampleIntensityWeight (beamfilters.hpp:150-190)
@@ -468,25 +469,25 @@ namespace {
         if (s.heel_weights) {
             // HeelFilter::sampleIntensityWeight (beamfilters.hpp:514-538)
             const Real energy = ph.energy;
-            int e_index = static_cast<int>((energy - s.heel_e_start + Real(0.5) * s.heel_e_step) / s.heel_e_step);
+            int e_index = static_cast<int>((energy - up<Real>(s.heel_e_start) + Real(0.5) * up<Real>(s.heel_e_step)) / up<Real>(s.heel_e_step));
             if (e_index >= s.heel_e_size || e_index < 0)
                 e_index = e_index < 0 ? 0 : s.heel_e_size - 1;
-            if (energy < s.heel_e_start)
+            if (energy < up<Real>(s.heel_e_start))
                 e_index = 0;
-            int a_index = static_cast<int>((phi - s.heel_a_start) / s.heel_a_step);
+            int a_index = static_cast<int>((phi - up<Real>(s.heel_a_start)) / up<Real>(s.heel_a_step));
             if (a_index >= s.heel_a_size || a_index < 0)
                 a_index = a_index < 0 ? 0 : s.heel_a_size - 1;
-            if (phi < s.heel_a_start)
+            if (phi < up<Real>(s.heel_a_start))
                 a_index = 0;
             const int w_index = e_index * s.heel_a_size + a_index;
             Real w;
             if (a_index < s.heel_a_size - 1) {
-                const Real a0 = s.heel_a_start + s.heel_a_step * a_index;
-                const Real a1 = s.heel_a_start + s.heel_a_step * (a_index + 1);
-                const Real w0 = __ldg(s.heel_weights + w_index), w1 = __ldg(s.heel_weights + w_index + 1);
+                const Real a0 = up<Real>(s.heel_a_start + s.heel_a_step * a_index);
+                const Real a1 = up<Real>(s.heel_a_start + s.heel_a_step * (a_index + 1));
+                const Real w0 = up<Real>(__ldg(s.heel_weights + w_index)), w1 = up<Real>(__ldg(s.heel_weights + w_index + 1));
                 w = w0 + (w1 - w0) * (phi - a0) / (a1 - a0);
             } else {
-                w = __ldg(s.heel_weights + w_index);
+                w = up<Real>(__ldg(s.heel_weights + w_index));
             }
             ph.weight *= w;
         }
@@ -495,7 +496,7 @@ namespace {
     template <class Real>
     __device__ __forceinline__ bool inside(const WorldParams& w, Real x, Real y, Real z)
     {
-        return (x > w.lo[0] && x < w.hi[0]) && (y > w.lo[1] && y < w.hi[1]) && (z > w.lo[2] && z < w.hi[2]);
+        return (x > up<Real>(w.lo[0]) && x < up<Real>(w.hi[0])) && (y > up<Real>(w.lo[1]) && y < up<Real>(w.hi[1])) && (z > up<Real>(w.lo[2]) && z < up<Real>(w.hi[2]));
     }
 
     // transportParticleToWorld (transport.hpp:702-728)
@@ -511,8 +512,8 @@ namespace {
         for (int i = 0; i < 3; ++i) {
             if (m_abs(dir[i]) > Real(N_ERROR_D)) {
                 const Real inv = Real(1.0) / dir[i];
-                const Real a0 = (w.lo[i] - pos[i]) * inv;
-                const Real an = (w.hi[i] - pos[i]) * inv;
+                const Real a0 = (up<Real>(w.lo[i]) - pos[i]) * inv;
+                const Real an = (up<Real>(w.hi[i]) - pos[i]) * inv;
                 amin = m_max(amin, m_min(a0, an));
                 amax = m_min(amax, m_max(a0, an));
             }
@@ -588,11 +589,11 @@ namespace {
     {
         if constexpr (PALETTE) {
             const PaletteEntry e = pal[raw.index];
-            density = e.density;
+            density = up<Real>(e.density);
             mat = static_cast<int>(e.code & 0xffu);
             measured = (e.code >> 8) != 0u;
         } else {
-            density = __uint_as_float(raw.v.x);
+            density = up<Real>(__uint_as_float(raw.v.x));
             mat = static_cast<int>(raw.v.y & 0xffu);
             measured = ((raw.v.y >> 8) & 0xffu) != 0u;
         }
@@ -610,7 +611,7 @@ namespace {
     // after each flight, to stop when few lanes were left, cost more than it saved.
     // CT 512 x 512 x 100 of 2e7 histories with bursts of 2 / 3 / 4 / 5: 2.49 / 2.42 / 2.41 /
     // 2.45 ms (2.52 voting); DX 160^3 of 5e6: 0.570 / 0.588 / 0.600 / 0.61 ms (0.587).
-    constexpr int START_BURST = 3;
+    constexpr int START_BURST = 3; // FP64: SHORT_BURST, each of its flights costs more
     constexpr int SHORT_BURST = 2, LONG_BURST = 4;
     constexpr uint32_t LONG_BURST_STOPS = 55; // per hundred flights, at most
 
@@ -717,15 +718,15 @@ namespace {
         const WorldParams& w = p.world;
         // the band intervals of the bounds are widened by 0.1 % on the host, which
         // covers the rounding here
-        s.band = min(max(m_floor_int((logE - g.band_log0) * g.band_inv_dlog), 0), g.bands - 1);
-        const Real fx = m_min(m_max(m_fma(s.ph.px, w.inv_spacing[0], -w.lo_inv[0]), Real(0.0)), w.dims_f[0] - Real(1.0));
-        const Real fy = m_min(m_max(m_fma(s.ph.py, w.inv_spacing[1], -w.lo_inv[1]), Real(0.0)), w.dims_f[1] - Real(1.0));
-        const Real fz = m_min(m_max(m_fma(s.ph.pz, w.inv_spacing[2], -w.lo_inv[2]), Real(0.0)), w.dims_f[2] - Real(1.0));
+        s.band = min(max(m_floor_int((logE - up<Real>(g.band_log0)) * up<Real>(g.band_inv_dlog)), 0), g.bands - 1);
+        const Real fx = m_min(m_max(m_fma(s.ph.px, up<Real>(w.inv_spacing[0]), -up<Real>(w.lo_inv[0])), Real(0.0)), up<Real>(w.dims_f[0]) - Real(1.0));
+        const Real fy = m_min(m_max(m_fma(s.ph.py, up<Real>(w.inv_spacing[1]), -up<Real>(w.lo_inv[1])), Real(0.0)), up<Real>(w.dims_f[1]) - Real(1.0));
+        const Real fz = m_min(m_max(m_fma(s.ph.pz, up<Real>(w.inv_spacing[2]), -up<Real>(w.lo_inv[2])), Real(0.0)), up<Real>(w.dims_f[2]) - Real(1.0));
         const uint32_t ix = static_cast<uint32_t>(fx), iy = static_cast<uint32_t>(fy), iz = static_cast<uint32_t>(fz);
         const uint32_t c = (iz >> g.shift[2]) * g.nxy + (iy >> g.shift[1]) * g.nx + (ix >> g.shift[0]);
         const float2 cell = __ldg(g.cells + (c * g.bands + s.band));
-        s.cinv = cell.x;
-        s.cR = cell.y;
+        s.cinv = up<Real>(cell.x);
+        s.cR = up<Real>(cell.y);
     }
 
     // Safe flight length in a cell outside the box of the denser cells (the cell
@@ -741,8 +742,8 @@ namespace {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const Real inv = Real(1.0) / d[a];
-            const Real t0 = (g.box_lo[a] - p[a]) * inv;
-            const Real t1 = (g.box_hi[a] - p[a]) * inv;
+            const Real t0 = (up<Real>(g.box_lo[a]) - p[a]) * inv;
+            const Real t1 = (up<Real>(g.box_hi[a]) - p[a]) * inv;
             tmin = m_max(tmin, m_min(t0, t1));
             tmax = m_min(tmax, m_max(t0, t1));
         }
@@ -856,7 +857,7 @@ namespace {
     __device__ __forceinline__ void roulette(LaneT<Real, Index>& s)
     {
         if (s.ph.energy * s.ph.weight < Real(ROULETTE_THRESHOLD_D)) {
-            if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D))
+            if (up<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D))
                 s.state = IDLE;
             else
                 s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
@@ -898,11 +899,11 @@ namespace {
         const Real eventProb = probInv * density * cinv;
         if (!FORCED || !measured) {
             // naive sampling (computeInteractions): the event runs in the interaction pass
-            if (static_cast<Real>(s.rng.uniform()) < eventProb) {
+            if (up<Real>(s.rng.uniform()) < eventProb) {
                 s.state = 1 + mat;
             } else if (s.armed) {
                 // virtual collision: Russian roulette (transport.hpp:684-694)
-                if (static_cast<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D)) {
+                if (up<Real>(s.rng.uniform()) < Real(ROULETTE_PROBABILITY_D)) {
                     s.state = IDLE;
                 } else {
                     s.ph.weight *= Real(1.0) / (Real(1.0) - Real(ROULETTE_PROBABILITY_D));
@@ -925,7 +926,7 @@ namespace {
             if (isfinite(forced_deposit)) {
                 score<FAST>(p, s.vidx, forced_deposit);
                 atomicAdd(&ws.forced_deposits, 1u);
-                if (static_cast<Real>(s.rng.uniform()) < eventProb * (Real(1.0) - photoProb)) {
+                if (up<Real>(s.rng.uniform()) < eventProb * (Real(1.0) - photoProb)) {
                     s.forced_wc = wc;
                     s.state = -1 - mat;
                 } else {
@@ -1005,7 +1006,7 @@ namespace {
             if (s.state == FLYING) {
                 // a flight drawn with the local majorant ends without a collision test
                 // where that majorant stops holding (truncated: drawn again from there)
-                const Real flight = -m_log2(static_cast<Real>(s.rng.uniform_open())) * (s.stepK * s.cinv);
+                const Real flight = -m_log2(up<Real>(s.rng.uniform_open())) * (s.stepK * s.cinv);
                 const Real R = m_abs(s.cR);
                 const bool truncated = flight > R;
                 if (truncated && s.cR < Real(0.0)) {
@@ -1021,9 +1022,9 @@ namespace {
                     // grid coordinates (p - lo) / spacing as one FMA each, rounded down; the photon
                     // is inside while all three lie in [0, dims) (one unsigned compare each: a
                     // negative or saturated conversion falls outside), which bounds the voxel index
-                    const uint32_t ix = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.px, w.inv_spacing[0], -w.lo_inv[0])));
-                    const uint32_t iy = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.py, w.inv_spacing[1], -w.lo_inv[1])));
-                    const uint32_t iz = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.pz, w.inv_spacing[2], -w.lo_inv[2])));
+                    const uint32_t ix = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.px, up<Real>(w.inv_spacing[0]), -up<Real>(w.lo_inv[0]))));
+                    const uint32_t iy = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.py, up<Real>(w.inv_spacing[1]), -up<Real>(w.lo_inv[1]))));
+                    const uint32_t iz = static_cast<uint32_t>(m_floor_int(m_fma(s.ph.pz, up<Real>(w.inv_spacing[2]), -up<Real>(w.lo_inv[2]))));
                     if (!(ix < w.dims[0] && iy < w.dims[1] && iz < w.dims[2])) {
                         s.state = IDLE;
                     } else {
@@ -1042,8 +1043,8 @@ namespace {
                             const MajorantGrid& g = p.majorant;
                             const uint32_t c = (iz >> g.shift[2]) * g.nxy + (iy >> g.shift[1]) * g.nx + (ix >> g.shift[0]);
                             const float2 cell = __ldg(g.cells + (c * g.bands + s.band));
-                            s.cinv = cell.x;
-                            s.cR = cell.y;
+                            s.cinv = up<Real>(cell.x);
+                            s.cR = up<Real>(cell.y);
                         }
                         if (!truncated) {
                             if constexpr (LEAN) {
@@ -1087,7 +1088,7 @@ namespace {
             } else {
                 type_shares(L, m, mat, E, p0, p01);
             }
-            const Real r3 = static_cast<Real>(s.rng.uniform());
+            const Real r3 = up<Real>(s.rng.uniform());
             photo = !forced && r3 < p0;
             compton = forced ? r3 * (Real(1.0) - p0) < p01 - p0 : (!photo && r3 < p01);
             if constexpr (MODEL == 1) {
@@ -1097,9 +1098,10 @@ namespace {
                     turn = false;
                 } else {
                     Real fe;
-                    const int row = table_row(m, E, fe);
+                    // in double the logarithm of the setup serves again
+                    const int row = table_row(m, SHARES ? s.logE * Real(2.30258509299404568402) : m_log(E), fe);
                     const float* tab = p.lut + (compton ? m.off_csf : m.off_ray) + (mat * m.tab_ne + row) * (m.tab_nu + 1);
-                    const Real x = table_quantile(tab, m.tab_nu, static_cast<Real>(s.rng.uniform()), fe);
+                    const Real x = table_quantile(tab, m.tab_nu, up<Real>(s.rng.uniform()), fe);
                     if (compton) {
                         Real e;
                         compton_from_fraction(E, x, e, cosA);
@@ -1169,8 +1171,9 @@ namespace {
         if (done) {
             s.state = FLYING;
             if (turn && ok) {
-                const Real phi = rng_azimuth<Real>(s.rng);
-                peturb(s.ph.dx, s.ph.dy, s.ph.dz, cosA, phi, !FAST && p.normalize_direction);
+                Real sin_phi, cos_phi;
+                rng_azimuth(s.rng, &sin_phi, &cos_phi);
+                peturb(s.ph.dx, s.ph.dy, s.ph.dz, cosA, sin_phi, cos_phi, !FAST && p.normalize_direction);
             }
             if (!ok) {
                 atomicAdd(&ws.overflows, 1u);
@@ -1290,7 +1293,7 @@ namespace {
             ws = WarpState {};
             const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
             ws.next = work_unit(p.work, unit, ws.end);
-            ws.burst = p.woodcock_burst > 0 ? p.woodcock_burst : START_BURST;
+            ws.burst = p.woodcock_burst > 0 ? p.woodcock_burst : (sizeof(Real) == 8 ? SHORT_BURST : START_BURST);
         }
         __syncwarp();
         LaneT<Real, typename VoxelRaw<PALETTE>::Index> s {};
@@ -1667,8 +1670,9 @@ namespace {
             else
                 ok = rayleigh_sample<MODEL>(L, m, ph.energy, material, rng, cosA);
             if (turn && ok) {
-                const float phi = rng_azimuth<float>(rng);
-                peturb(ph.dx, ph.dy, ph.dz, cosA, phi);
+                float sin_phi, cos_phi;
+                rng_azimuth(rng, &sin_phi, &cos_phi);
+                peturb(ph.dx, ph.dy, ph.dz, cosA, sin_phi, cos_phi);
             }
             const float len = sqrtf(ph.dx * ph.dx + ph.dy * ph.dy + ph.dz * ph.dz);
             out_cos[i] = ok ? (len > 0 ? ph.dz / len : 1.0f) : 2.0f;
