@@ -147,29 +147,32 @@ struct TransportParams {
     MajorantGrid majorant;
 };
 
-// Work item of the batched kernel: histories [first, first + count) of job `job`.
+// A job of a batch as the batched kernel's warps look for work: jobs of one model lie
+// in a row, `first` is the position of the job's first history among theirs.
 struct BatchItem {
     uint32_t job;
-    uint32_t count;
+    uint32_t pad;
     uint64_t first;
+    uint64_t histories;
+    JobCounters* counters; // next_history: the job's histories handed out
 };
 
 // Per-batch control block in device memory, written by one host-to-device copy
 // before the batch kernels start: the kernels' own arguments never change, so
 // one instantiated CUDA graph serves every batch of an engine.
 struct BatchControl {
-    unsigned long long next_item[4]; // work-queue heads, one per correction model (start at zero)
-    uint64_t item_base[4];           // first item of each model in the item array
-    uint64_t n_items[4];             // items of each model
+    uint64_t item_base[4]; // first job of each correction model in the item array
+    uint64_t n_items[4];   // jobs of each model
+    uint64_t histories[4]; // of all of them
+    uint64_t chunk;        // histories that a warp takes at once, a multiple of 32
     int regen_threshold;
     int interact_threshold;
-    int pad[2];
 };
 
 struct BatchParams {
     const TransportParams* jobs;
     const BatchItem* items;
-    BatchControl* control;
+    const BatchControl* control;
 };
 
 // Launchers (defined in transport_kernels.cu).

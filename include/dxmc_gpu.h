@@ -375,9 +375,9 @@ void dxmc_gpu_job_free(dxmc_job* job);
 
 /* ---- batches: many jobs in one persistent launch ---------------------------- */
 /* No counterpart in the reference (which runs one source at a time).  Every
- * job keeps its own world, LUT, source tables and tallies; the jobs are cut
- * into work items on a device-side queue that one persistent kernel launch
- * (per correction model) drains.  A job's tallies are the same whether it runs
+ * job keeps its own world, LUT, source tables and tallies; the blocks of one
+ * persistent kernel launch (per correction model) take histories from the jobs,
+ * one job at a time.  A job's tallies are the same whether it runs
  * alone or in a batch (each history has its own random stream). */
 typedef struct dxmc_batch dxmc_batch;
 typedef struct dxmc_batch_entry {
@@ -395,7 +395,7 @@ typedef struct dxmc_batch_options {
     int32_t chains;             /* concurrent mode: parallel chains (1..8); 0: 2 */
     int32_t regen_threshold;    /* persistent mode: refill idle lanes once this many are idle (1..32); 0: default */
     int32_t interact_threshold; /* persistent mode: interaction passes once this many lanes wait (1..32); 0: default */
-    int32_t item_histories;     /* persistent mode: histories per work item; 0: automatic (256..8192) */
+    int32_t item_histories;     /* persistent mode: histories a warp takes at once; 0: 128 */
     int32_t pad;
 } dxmc_batch_options;
 /* Non-blocking.  At most 4096 jobs per batch; `options` may be NULL.
