@@ -205,8 +205,8 @@ struct dxmc_gpu_ctx {
     // do not wait for those of a job that still runs
     static constexpr int ASYNC_STREAMS = 4;
     cudaStream_t async_streams[ASYNC_STREAMS] {};
+    cudaStream_t copy_streams[ASYNC_STREAMS] {}; // copies of large results, beside the later pieces' kernels
     int next_async = 0;
-    cudaStream_t piece_stream = nullptr; // every other piece of a large result
     // world and table uploads: their copies and host waits do not queue behind
     // the jobs on the context stream (uploading the next world overlaps a job)
     cudaStream_t upload_stream = nullptr;
@@ -849,10 +849,11 @@ try {
     int least_priority = 0, greatest_priority = 0;
     cudaDeviceGetStreamPriorityRange(&least_priority, &greatest_priority);
     const int result_priority = std::min(least_priority, greatest_priority + 1);
-    bool streams = cudaStreamCreateWithPriority(&ctx->result_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess
-        && cudaStreamCreateWithPriority(&ctx->piece_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess;
+    bool streams = cudaStreamCreateWithPriority(&ctx->result_stream, cudaStreamNonBlocking, result_priority) == cudaSuccess;
     for (cudaStream_t& r : ctx->async_streams)
         streams = streams && cudaStreamCreateWithPriority(&r, cudaStreamNonBlocking, result_priority) == cudaSuccess;
+    for (cudaStream_t& r : ctx->copy_streams)
+        streams = streams && cudaStreamCreateWithFlags(&r, cudaStreamNonBlocking) == cudaSuccess;
     streams = streams && cudaStreamCreateWithPriority(&ctx->upload_stream, cudaStreamNonBlocking, greatest_priority) == cudaSuccess;
     if (!streams) {
         destroy_ctx_streams(ctx);
@@ -2619,7 +2620,10 @@ void wait_unused(dxmc_gpu_ctx* ctx, const Usage& u)
 
 void destroy_ctx_streams(dxmc_gpu_ctx* ctx)
 {
-    for (cudaStream_t st : { ctx->stream, ctx->result_stream, ctx->piece_stream, ctx->upload_stream })
+    for (cudaStream_t st : { ctx->stream, ctx->result_stream, ctx->upload_stream })
+        if (st)
+            cudaStreamDestroy(st);
+    for (cudaStream_t st : ctx->copy_streams)
         if (st)
             cudaStreamDestroy(st);
     for (cudaStream_t st : ctx->async_streams)
@@ -2631,7 +2635,8 @@ void sync_ctx_streams(dxmc_gpu_ctx* ctx)
 {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->result_stream);
-    cudaStreamSynchronize(ctx->piece_stream);
+    for (cudaStream_t r : ctx->copy_streams)
+        cudaStreamSynchronize(r);
     for (cudaStream_t r : ctx->async_streams)
         if (r)
             cudaStreamSynchronize(r);
@@ -2747,22 +2752,24 @@ dev::JobCounters* mapped_counters(const dxmc_job* j)
     return reinterpret_cast<dev::JobCounters*>(reinterpret_cast<unsigned char*>(j->cancel_dev) + 16);
 }
 
-// Results of a finished job into pageable host arrays: pieces go over the link into
-// page-locked blocks (written by the post-processing itself) while a few threads copy
-// earlier pieces to the caller's arrays.  A copy straight to pageable memory runs at the
+// Results of a finished job into pageable host arrays: one post-processing kernel writes
+// them to device memory, and pieces go over the link into page-locked blocks while a few
+// threads copy earlier pieces to the caller's arrays.  (A kernel per piece would wait, each
+// time, for another job's transport kernel that has taken the SMs in between.)  A copy straight to pageable memory runs at the
 // speed of one thread that also takes the page faults of arrays not touched before: 28 ms
 // for the 150 MB of a 333 x 287 x 77 grid, 5 ms this way.
 constexpr uint64_t PAGEABLE_PIECE = 48 * 1024; // voxels: 960 KB of double results per block
 constexpr int PAGEABLE_THREADS = 8;
 constexpr uint64_t SMALL_PAGEABLE_BYTES = 16ull << 20; // 5 MB: 0.23 ms by the driver, 0.41 ms by the threads
-constexpr uint64_t DIRECT_RESULT_BYTES = 16ull << 20; // written over the link by the kernel: 0.09 ms at most
 constexpr uint64_t PIECED_RESULT_BYTES = 64ull << 20;
+constexpr uint64_t RESULT_PIECES = 4; // 629 MB: 0.6 ms less than in one
+constexpr uint64_t DIRECT_RESULT_BYTES = 16ull << 20; // written over the link by the kernel: 0.09 ms at most
 
 // Blocks and threads of such a transfer.  `locked`: the caller holds the context's mutex.
-// enqueue(k, block, device address, stream) queues piece k into a block, consume(k, block)
+// enqueue(k, block, stream) queues piece k into a block, consume(k, block)
 // takes it from there; each thread has a block of its own and takes the next piece.
 cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, size_t block_bytes, const cudaStream_t* streams, int n_streams,
-    const std::function<cudaError_t(uint64_t, unsigned char*, unsigned char*, cudaStream_t)>& enqueue,
+    const std::function<cudaError_t(uint64_t, unsigned char*, cudaStream_t)>& enqueue,
     const std::function<void(uint64_t, const unsigned char*)>& consume)
 {
     const int cores = static_cast<int>(std::max(1u, std::thread::hardware_concurrency() / 2));
@@ -2770,7 +2777,6 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
     struct Block {
         void* host = nullptr;
         size_t cls = 0;
-        unsigned char* dev = nullptr;
         cudaEvent_t done = nullptr;
     };
     std::vector<Block> blocks(threads);
@@ -2785,8 +2791,6 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
         for (Block& b : blocks) {
             if (e == cudaSuccess)
                 e = ctx->staging.take(block_bytes, &b.host, &b.cls);
-            if (e == cudaSuccess && !mapped_host(static_cast<unsigned char*>(b.host), b.dev))
-                e = cudaErrorInvalidValue;
             if (e == cudaSuccess)
                 e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
         }
@@ -2798,12 +2802,13 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
         cudaSetDevice(ctx->device);
         cudaStream_t s = streams[t % n_streams];
         for (uint64_t k; failed.load() == cudaSuccess && (k = next.fetch_add(1)) < pieces;) {
-            cudaError_t we = enqueue(k, static_cast<unsigned char*>(b.host), b.dev, s);
+            cudaError_t we = enqueue(k, static_cast<unsigned char*>(b.host), s);
             if (we == cudaSuccess)
                 we = cudaEventRecord(b.done, s);
             if (we == cudaSuccess)
                 we = cudaEventSynchronize(b.done);
             if (we != cudaSuccess) {
+                cudaStreamSynchronize(s); // what was queued still writes the block
                 failed.store(static_cast<int>(we));
                 return;
             }
@@ -2835,17 +2840,31 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
     return e;
 }
 
-cudaError_t results_to_pageable(dxmc_job* j, const ResultRequest& r, double* dose, double* variance, uint32_t* counts)
+// Post-processed results in device memory, complete once `ready` has happened.
+struct StagedResults {
+    unsigned char* dose = nullptr;
+    unsigned char* variance = nullptr;
+    unsigned char* counts = nullptr;
+    cudaEvent_t ready = nullptr;
+};
+
+cudaError_t results_to_pageable(dxmc_job* j, const StagedResults& r, double* dose, double* variance, uint32_t* counts)
 {
     const uint64_t nv = j->world->params.n_voxels;
     constexpr size_t VAR_AT = PAGEABLE_PIECE * sizeof(double), COUNT_AT = 2 * VAR_AT;
     return transfer_pieces(
         j->ctx, false, (nv + PAGEABLE_PIECE - 1) / PAGEABLE_PIECE, COUNT_AT + PAGEABLE_PIECE * sizeof(uint32_t), j->ctx->async_streams,
         dxmc_gpu_ctx::ASYNC_STREAMS,
-        [&](uint64_t k, unsigned char*, unsigned char* dev, cudaStream_t s) {
-            const uint64_t first = k * PAGEABLE_PIECE;
-            return post_process(j, r, first, std::min(PAGEABLE_PIECE, nv - first), dose ? dev : nullptr, variance ? dev + VAR_AT : nullptr,
-                counts ? reinterpret_cast<uint32_t*>(dev + COUNT_AT) : nullptr, nullptr, s);
+        [&](uint64_t k, unsigned char* h, cudaStream_t s) {
+            const uint64_t first = k * PAGEABLE_PIECE, n = std::min(PAGEABLE_PIECE, nv - first);
+            cudaError_t e = cudaStreamWaitEvent(s, r.ready, 0);
+            if (e == cudaSuccess && dose)
+                e = cudaMemcpyAsync(h, r.dose + first * sizeof(double), n * sizeof(double), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess && variance)
+                e = cudaMemcpyAsync(h + VAR_AT, r.variance + first * sizeof(double), n * sizeof(double), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess && counts)
+                e = cudaMemcpyAsync(h + COUNT_AT, r.counts + first * sizeof(uint32_t), n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            return e;
         },
         [&](uint64_t k, const unsigned char* h) {
             const uint64_t first = k * PAGEABLE_PIECE, n = std::min(PAGEABLE_PIECE, nv - first);
@@ -2869,7 +2888,7 @@ cudaError_t energy_of_records(dxmc_job* j, uint32_t copies, double* energy)
     for (uint32_t c = 0; c < copies && e == cudaSuccess; ++c)
         e = transfer_pieces(
             j->ctx, true, (nv + PIECE - 1) / PIECE, PIECE * sizeof(dev::TallyRecord), &j->ctx->result_stream, 1,
-            [&](uint64_t k, unsigned char* h, unsigned char*, cudaStream_t s) {
+            [&](uint64_t k, unsigned char* h, cudaStream_t s) {
                 const uint64_t first = k * PIECE;
                 return cudaMemcpyAsync(h, j->records + c * nv + first, std::min(PIECE, nv - first) * sizeof(dev::TallyRecord), cudaMemcpyDeviceToHost, s);
             },
@@ -2896,6 +2915,8 @@ try {
     const ResultRequest request { output_mode, calibration, false };
     cudaEvent_t done = nullptr;
     bool pageable = false;
+    unsigned char* stage = nullptr;
+    StagedResults staged;
     {
         // queue post-processing and copies on the result stream under the lock, wait without it
         std::lock_guard<std::mutex> lock(ctx->mutex);
@@ -2913,22 +2934,24 @@ try {
             && (!n_events || mapped_host(n_events, m_events));
         const uint64_t bytes = ((dose ? nv : 0) + (variance ? nv : 0)) * sizeof(double) + (n_events ? nv * sizeof(uint32_t) : 0);
         pageable = wanted && !mapped && bytes > SMALL_PAGEABLE_BYTES;
-        if (wanted && !mapped && !pageable) {
-            // small pageable arrays: the driver's own copies
-            unsigned char* stage = nullptr;
+        if (wanted && !mapped) {
             DXMC_CUDA(ctx, cudaMemcpyAsync(host_counters(j), j->counters, sizeof(dev::JobCounters), cudaMemcpyDeviceToHost, s));
             DXMC_CUDA(ctx, pool_alloc(ctx, &stage, bytes, s));
-            unsigned char* d_var = stage + (dose ? nv * sizeof(double) : 0);
-            unsigned char* d_counts = d_var + (variance ? nv * sizeof(double) : 0);
-            cudaError_t e = post_process(j, request, 0, nv, dose ? stage : nullptr, variance ? d_var : nullptr,
-                n_events ? reinterpret_cast<uint32_t*>(d_counts) : nullptr, nullptr, s);
-            if (e == cudaSuccess && dose)
-                e = cudaMemcpyAsync(dose, stage, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess && variance)
-                e = cudaMemcpyAsync(variance, d_var, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess && n_events)
-                e = cudaMemcpyAsync(n_events, d_counts, nv * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-            cudaFreeAsync(stage, s);
+            staged.dose = stage;
+            staged.variance = stage + (dose ? nv * sizeof(double) : 0);
+            staged.counts = staged.variance + (variance ? nv * sizeof(double) : 0);
+            cudaError_t e = post_process(j, request, 0, nv, dose ? staged.dose : nullptr, variance ? staged.variance : nullptr,
+                n_events ? reinterpret_cast<uint32_t*>(staged.counts) : nullptr, nullptr, s);
+            if (!pageable) { // small arrays: the driver's own copies
+                if (e == cudaSuccess && dose)
+                    e = cudaMemcpyAsync(dose, staged.dose, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
+                if (e == cudaSuccess && variance)
+                    e = cudaMemcpyAsync(variance, staged.variance, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
+                if (e == cudaSuccess && n_events)
+                    e = cudaMemcpyAsync(n_events, staged.counts, nv * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            }
+            if (!pageable || e != cudaSuccess)
+                cudaFreeAsync(stage, s);
             if (e != cudaSuccess)
                 return cuda_fail(ctx, e, "result post-processing");
         } else if (mapped && j->records) {
@@ -2941,19 +2964,32 @@ try {
             if (e != cudaSuccess)
                 return cuda_fail(ctx, e, "result post-processing");
         }
-        DXMC_CUDA(ctx, cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
-        const cudaError_t e = cudaEventRecord(done, s);
+        cudaError_t e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(done, s);
         if (e != cudaSuccess) {
-            cudaEventDestroy(done);
+            if (pageable)
+                cudaFreeAsync(stage, s);
+            if (done)
+                cudaEventDestroy(done);
             return cuda_fail(ctx, e, "result copy");
         }
+        staged.ready = done;
     }
-    cudaError_t e = pageable ? results_to_pageable(j, request, dose, variance, n_events) : cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    try {
+        if (pageable)
+            e = results_to_pageable(j, staged, dose, variance, n_events);
+    } catch (const std::bad_alloc&) {
+        e = cudaErrorMemoryAllocation;
+    }
     const cudaError_t de = cudaEventSynchronize(done);
     if (e == cudaSuccess)
         e = de;
     cudaEventDestroy(done);
     std::lock_guard<std::mutex> lock(ctx->mutex);
+    if (pageable)
+        cudaFreeAsync(stage, ctx->result_stream); // its copies have ended
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "result copy");
     const dev::JobCounters c = *host_counters(j);
@@ -3075,7 +3111,6 @@ try {
     const bool direct = j->records && (dose || variance || n_events) && nv * per_voxel <= DIRECT_RESULT_BYTES
         && (!dose || mapped_host(dose, m_dose)) && (!variance || mapped_host(variance, m_var)) && (!n_events || mapped_host(n_events, m_events));
     unsigned char* stage = nullptr;
-    cudaEvent_t other_done = nullptr;
     cudaError_t e = cudaSuccess;
     if (direct) {
         e = post_process(j, request, 0, nv, m_dose, m_var, m_events, mapped_counters(j), s);
@@ -3083,42 +3118,39 @@ try {
         e = cudaMemcpyAsync(host_counters(j), j->counters, sizeof(dev::JobCounters), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && per_voxel)
             e = pool_alloc(ctx, &stage, nv * per_voxel, s);
-        // large results in pieces on two streams in turn: one piece's post-processing
-        // runs beside the copies of the piece before it
-        const uint64_t pieces = nv * per_voxel > PIECED_RESULT_BYTES ? 8 : 1;
-        cudaStream_t streams[2] = { s, s };
-        if (pieces > 1) {
-            streams[1] = ctx->piece_stream;
-            if (e == cudaSuccess)
-                e = cudaEventCreateWithFlags(&other_done, cudaEventDisableTiming);
-            if (e == cudaSuccess)
-                e = cudaEventRecord(other_done, s); // the stage exists, the job has ended
-            if (e == cudaSuccess)
-                e = cudaStreamWaitEvent(streams[1], other_done, 0);
-        }
-        const uint64_t piece = (nv + pieces - 1) / pieces;
-        unsigned char* d_dose = stage;
         unsigned char* d_var = stage + (dose ? nv * elem : 0);
         uint32_t* d_counts = reinterpret_cast<uint32_t*>(stage + ((dose ? nv : 0) + (variance ? nv : 0)) * elem);
-        for (uint64_t k = 0, first = 0; first < nv && e == cudaSuccess; ++k, first += piece) {
+        // large results in pieces: one piece's post-processing runs beside the copies of the
+        // piece before it.  The kernels follow one another directly on `s`, so that no
+        // transport kernel comes between them; the copies wait for theirs on another stream.
+        const uint64_t pieces = nv * per_voxel > PIECED_RESULT_BYTES ? RESULT_PIECES : 1;
+        const cudaStream_t cs = pieces > 1 ? ctx->copy_streams[at] : s;
+        const uint64_t piece = (nv + pieces - 1) / pieces;
+        cudaEvent_t ready = nullptr;
+        if (e == cudaSuccess && pieces > 1)
+            e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+        for (uint64_t first = 0; first < nv && e == cudaSuccess; first += piece) {
             const uint64_t n = std::min(piece, nv - first);
-            cudaStream_t ps = streams[k % 2];
             if (per_voxel)
-                e = post_process(j, request, first, n, dose ? d_dose + first * elem : nullptr, variance ? d_var + first * elem : nullptr,
-                    counts_staged ? d_counts + first : nullptr, nullptr, ps);
+                e = post_process(j, request, first, n, dose ? stage + first * elem : nullptr, variance ? d_var + first * elem : nullptr,
+                    counts_staged ? d_counts + first : nullptr, nullptr, s);
+            if (e == cudaSuccess && ready)
+                e = cudaEventRecord(ready, s);
+            if (e == cudaSuccess && ready)
+                e = cudaStreamWaitEvent(cs, ready, 0);
             if (e == cudaSuccess && dose)
-                e = cudaMemcpyAsync(static_cast<unsigned char*>(dose) + first * elem, d_dose + first * elem, n * elem, cudaMemcpyDeviceToHost, ps);
+                e = cudaMemcpyAsync(static_cast<unsigned char*>(dose) + first * elem, stage + first * elem, n * elem, cudaMemcpyDeviceToHost, cs);
             if (e == cudaSuccess && variance)
-                e = cudaMemcpyAsync(static_cast<unsigned char*>(variance) + first * elem, d_var + first * elem, n * elem, cudaMemcpyDeviceToHost, ps);
+                e = cudaMemcpyAsync(static_cast<unsigned char*>(variance) + first * elem, d_var + first * elem, n * elem, cudaMemcpyDeviceToHost, cs);
             if (e == cudaSuccess && n_events)
-                e = cudaMemcpyAsync(n_events + first, counts_staged ? d_counts + first : j->n_events + first, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, ps);
+                e = cudaMemcpyAsync(n_events + first, counts_staged ? d_counts + first : j->n_events + first, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs);
         }
-        if (other_done) {
+        if (ready) {
             if (e == cudaSuccess)
-                e = cudaEventRecord(other_done, streams[1]);
+                e = cudaEventRecord(ready, cs);
             if (e == cudaSuccess)
-                e = cudaStreamWaitEvent(s, other_done, 0);
-            cudaEventDestroy(other_done); // released once it has completed
+                e = cudaStreamWaitEvent(s, ready, 0);
+            cudaEventDestroy(ready); // released once it has completed
         }
     }
     if (stage)
