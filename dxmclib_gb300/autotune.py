@@ -14,7 +14,7 @@ model):
 * ``blocks_per_sm`` -- resident blocks per SM (occupancy);
 * ``block_size`` -- threads per block (128 or 256);
 * ``woodcock_burst`` -- Woodcock steps a lane may take per loop iteration before
-  the warp checks for refills and interactions again.
+  the warp checks for refills and interactions again (0: each warp chooses).
 
 For a job class (correction model, grid size in factors of 8, number of
 materials, maximum energy in 20 keV bins) the tuner times a sample of the job -- an even

@@ -139,7 +139,7 @@ struct TransportParams {
     int lut_in_smem;
     int regen_threshold;    // refill finished lanes once at least this many are idle (1..32)
     int interact_threshold; // run the interaction passes once at least this many lanes wait (1..32)
-    int woodcock_burst;     // Woodcock steps a lane may take per loop iteration (1..64)
+    int woodcock_burst;     // Woodcock steps a lane may take per loop iteration (1..64); 0: chosen by the warp as it goes
     int normalize_direction; // 1: unit scattering axis in peturb (normalised physics), 0: the reference's
     int precision;          // 0: FP32 transport; 1: FP64 everywhere (position, direction, energy, LUT, sampling)
     int pad_precision;

@@ -2,9 +2,9 @@
 //
 // One persistent launch per job: every lane owns one photon history at a
 // time and, inside a warp-synchronous loop, takes a burst of Woodcock steps per
-// iteration.  Lanes whose history ended take the next history id from a
-// warp-local pool that one lane refills from a global work queue, so warps
-// stay full until the job runs dry.  Physics follows DXMClib's
+// iteration.  Lanes whose history ended take a photon from a pool that the
+// whole warp fills together, so warps stay full until the job runs dry.
+// Physics follows DXMClib's
 // Transport<T> (include/dxmc/transport.hpp) function by function; each
 // device function names the reference lines it restates.
 #include "transport.cuh"
@@ -1242,12 +1242,15 @@ namespace {
     // enough lanes want it.  Idle lanes take photons from the warp's pool, which all 32
     // lanes fill together; new photons and new energies are set up together; the lanes
     // then fly a burst; and once enough of them wait for an event the interactions run in
-    // one pass.  64 registers (four blocks of 256 threads per SM; 48 or 40 registers
-    // spilled and ran 20 to 30 % slower); what belongs to the warp lives in shared memory.
-    // Sampling in place and the box test in the flight loop before; now, kernel alone:
-    // CT 512 x 512 x 200 of 1e8 histories 13.4 -> 12.7 ms, DX 160^3 of 5e6 0.753 -> 0.609 ms,
-    // CTDI phantom of 1e7 with forced scoring 1.29 -> 1.12 ms, DX 96^3 of 1e6 in FP64
-    // 6.4 -> 4.5 ms (two blocks per SM: about twice the registers).
+    // one pass.  Four blocks per SM, of 288 threads where 56 registers are enough and of 256
+    // with 64 (see transport_block; 48 or 40 registers spilled and ran 20 to 30 % slower);
+    // what belongs to the warp lives in shared memory, the LUT too (read through L1: CT 8 %,
+    // DX 12 %, IA 4 % slower).  Against photons sampled in place, the box test and the
+    // attenuation in the flight loop and a vote after each flight, kernel alone: CT
+    // 512 x 512 x 200 of 1e8 histories 13.4 -> 11.4 ms, DX 160^3 of 5e6 0.753 -> 0.549 ms,
+    // with impulse approximation (127^3, 4e6) 1.85 -> 1.13 ms, CTDI phantom of 1e7 with
+    // forced scoring 1.29 -> 1.01 ms, DX 96^3 of 1e6 in FP64 6.4 -> 4.3 ms (two blocks per
+    // SM: about twice the registers; FP64 pipe 86 % busy).
     template <class Real, int MODEL, bool PALETTE, bool FORCED, bool FAST>
     __global__ void __launch_bounds__(transport_block(FAST, FORCED, PALETTE, MODEL), sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
     {

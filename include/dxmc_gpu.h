@@ -243,7 +243,7 @@ typedef struct dxmc_job dxmc_job;
 
 typedef struct dxmc_gpu_options {
     int32_t device;          /* CUDA device ordinal */
-    int32_t block_size;      /* threads per block, 0 = default (256) */
+    int32_t block_size;      /* threads per block, 0 = default (256; 288 where 56 registers a thread are enough) */
     int32_t blocks_per_sm;   /* resident blocks per SM, 0 = occupancy-derived */
     int32_t tally_mode;      /* DXMC_TALLY_* */
     uint64_t memory_budget;  /* admission budget in bytes, 0 = 90% of free memory */
@@ -324,7 +324,7 @@ typedef struct dxmc_job_desc {
     int32_t interact_threshold;         /* interaction passes once this many lanes wait (1..32) */
     int32_t blocks_per_sm;              /* resident blocks per SM (1..occupancy limit) */
     int32_t queue_log2_chunk;           /* photon queue chunk 2^n; -1 = photons generated in the kernel */
-    int32_t woodcock_burst;             /* Woodcock steps a lane may take per loop iteration (1..64) */
+    int32_t woodcock_burst;             /* Woodcock steps a lane may take per loop iteration (1..64); default: chosen by each warp */
     int32_t block_size;                 /* threads per block of the transport kernel: 128 or 256 */
     int32_t tracking;                   /* DXMC_TRACKING_*; 0 = the context's */
     int32_t direction;                  /* DXMC_DIRECTION_* */

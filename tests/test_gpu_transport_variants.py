@@ -74,7 +74,8 @@ def test_usual_and_general_kernels_agree(gpu_ctx, model, materials, measured, la
 
 @pytest.mark.parametrize("histories", [1, 31, 33, 155_647, 155_649, 311_297, 500_003, 4_000_037])
 def test_work_split_takes_every_history_once(gpu_ctx, histories):
-    """155 648 histories are one round of 32 for 152 SMs of four eight-warp blocks."""
+    """155 648 histories are one round of 32 for 152 SMs of four eight-warp blocks (of
+    nine warps: 175 104)."""
     import dxmclib_gb300 as dx
     w = _world(2, False, np.random.default_rng(2))
     dworld = dx.DeviceWorld(gpu_ctx, w)
