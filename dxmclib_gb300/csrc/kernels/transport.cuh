@@ -2,6 +2,7 @@
 #pragma once
 
 #include "device_common.cuh"
+#include "work_split.hpp"
 
 namespace dxmc_gb300::dev {
 
@@ -107,14 +108,6 @@ struct alignas(32) TallyRecord {
     uint64_t pad1;
 };
 static_assert(sizeof(TallyRecord) == 32, "one tally record per 32-byte sector");
-
-// A job's ids in units that a warp takes at a time: `large_units` of `large` ids, then
-// units of `small` (both multiples of 32).
-struct WorkSplit {
-    uint64_t large_units = 0;
-    uint32_t large = 256;
-    uint32_t small = 32;
-};
 
 struct TransportParams {
     WorldParams world;

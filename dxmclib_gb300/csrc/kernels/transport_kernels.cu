@@ -790,15 +790,13 @@ namespace {
             s.state = IDLE;
     }
 
-    // The ids of one unit of a job's work (see WorkSplit); a unit past the end starts at
-    // or after the job's last id.
-    __device__ __forceinline__ uint64_t work_unit(const WorkSplit& w, uint64_t unit, uint64_t& end)
-    {
-        const bool large = unit < w.large_units;
-        const uint64_t first = large ? unit * w.large : w.large_units * w.large + (unit - w.large_units) * w.small;
-        end = first + (large ? w.large : w.small);
-        return first;
-    }
+    // The lanes of a warp for next_ids.
+    struct DeviceWarp {
+        __device__ __forceinline__ bool leader() const { return (threadIdx.x & 31) == 0; }
+        __device__ __forceinline__ void sync() const { __syncwarp(); }
+        __device__ __forceinline__ uint64_t broadcast(uint64_t v) const { return __shfl_sync(FULL_MASK, v, 0); }
+        __device__ __forceinline__ uint64_t fetch_add(unsigned long long* head) const { return atomicAdd(head, 1ull); }
+    };
 
     // Photons sampled ahead for one warp (shared memory, one row per field).  All 32
     // lanes sample together, whatever their own photons do; idle lanes then take photons
@@ -1310,24 +1308,13 @@ namespace {
                 while (need) {
                     const int pooled = ws.pooled;
                     if (pooled == 0) {
-                        uint64_t next = ws.next;
-                        if (next >= ws.end) {
-                            // a unit of the job is done: the job's progress, and the next unit
-                            if (ws.histories >= PUBLISH_HISTORIES)
-                                add_counters(ws, p.counters);
-                            if (lane == 0) {
-                                const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
-                                unsigned long long* head = use_queue ? &p.counters->next_photon : &p.counters->next_history;
-                                const uint64_t unit = warps + atomicAdd(head, 1ull);
-                                uint64_t end;
-                                next = work_unit(p.work, unit, end);
-                                ws.end = end;
-                                // the host's flag costs a read over the link: not at every small unit
-                                if (unit < p.work.large_units && p.cancel && *p.cancel)
-                                    next = source_total;
-                            }
-                            next = __shfl_sync(FULL_MASK, next, 0);
-                        }
+                        // a unit of the job is done: the job's progress, and the next unit
+                        if (ws.next >= ws.end && ws.histories >= PUBLISH_HISTORIES)
+                            add_counters(ws, p.counters);
+                        const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
+                        DeviceWarp self;
+                        const uint64_t next = next_ids(self, ws, p.work, warps, use_queue ? &p.counters->next_photon : &p.counters->next_history,
+                            source_total, [&p] { return p.cancel && *p.cancel; });
                         if (next >= source_total) {
                             exhausted = true;
                             break;
@@ -1505,6 +1492,7 @@ namespace {
                             if (p.woodcock_burst == 0 && ws.steps >= 256)
                                 ws.burst = (ws.deposits + ws.forced_deposits + ws.histories) * 100 > ws.steps * LONG_BURST_STOPS ? SHORT_BURST : LONG_BURST;
                         }
+                        __syncwarp(); // the other lanes read the burst next
                         if (mine)
                             take_history(s, p, next + rank);
                         next += __popc(taken);

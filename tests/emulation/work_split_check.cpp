@@ -1,0 +1,66 @@
+// A warp's way through a job's work units (next_ids), with lanes that advance one at a time.
+#include "kernels/work_split.hpp"
+#include "warp_lanes.hpp"
+
+#include <algorithm>
+
+using namespace dxmc_gb300;
+
+namespace {
+
+struct Ids {
+    std::uint64_t next = 0, end = 0;
+};
+
+int failures = 0;
+void check(bool ok, const char* what)
+{
+    if (!ok) {
+        std::printf("FAIL %s\n", what);
+        ++failures;
+    }
+}
+
+// One warp takes all units of a job of `total` ids: every id once, all lanes the same.
+void all_ids_once(const WorkSplit& work, std::uint64_t total, bool ascending)
+{
+    Ids ids;
+    ids.next = work_unit(work, 0, ids.end);
+    unsigned long long head = 0;
+    std::vector<int> taken(total, 0);
+    emulation::Warp warp;
+    const bool converged = warp.run(
+        [&](emulation::Warp& w, int lane) {
+            while (true) {
+                const std::uint64_t next = next_ids(w, ids, work, 1, &head, total, [] { return false; });
+                if (next >= total)
+                    break;
+                if (next + lane < total)
+                    ++taken[next + lane];
+                w.sync(); // the votes over the sampled photons
+                if (w.leader())
+                    ids.next = next + 32;
+                w.sync();
+            }
+        },
+        ascending);
+    check(converged, "lanes meet at the same collective");
+    check(std::all_of(taken.begin(), taken.end(), [](int n) { return n == 1; }), "every id is taken once");
+}
+
+} // namespace
+
+int main()
+{
+    for (const bool ascending : { true, false })
+        for (const std::uint64_t total : { 1u, 31u, 32u, 33u, 700u, 1500u }) {
+            WorkSplit work; // small units only
+            all_ids_once(work, total, ascending);
+            work.large_units = 2; // two large units, then small ones
+            all_ids_once(work, total, ascending);
+            work.small = 64;
+            all_ids_once(work, total, ascending);
+        }
+    std::printf(failures ? "%d checks failed\n" : "ok\n", failures);
+    return failures ? 1 : 0;
+}

@@ -1,0 +1,22 @@
+"""CPU tests of warp-level device code with the lanes of a warp advancing one at a
+time (tests/emulation): the code is compiled for the host from the kernels' own
+headers."""
+from __future__ import annotations
+
+import subprocess
+from pathlib import Path
+
+REPO = Path(__file__).resolve().parents[1]
+
+
+def _run(name, tmp_path):
+    exe = tmp_path / name
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", f"-I{REPO / 'dxmclib_gb300' / 'csrc'}", f"-I{REPO / 'tests' / 'emulation'}",
+                        str(REPO / "tests" / "emulation" / f"{name}.cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_work_units_are_taken_whatever_the_order_of_the_lanes(tmp_path):
+    _run("work_split_check", tmp_path)
