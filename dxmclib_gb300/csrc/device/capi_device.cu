@@ -1286,13 +1286,9 @@ try {
                 o[5 + k] = static_cast<float>(c.line_probabilities[k]);
                 o[8 + k] = static_cast<float>(c.line_energies[k]);
             }
-            // the partial sums, in the order and precision of the kernels'
-            float* sums = img.data() + m.off_shell_sums + mat * dev::SHELL_SUM_FLOATS;
-            const float electrons = o[2] > 0.0f ? o[1] : 0.0f;
-            sums[s] = s > 0 ? sums[s - 1] + electrons : electrons;
-            sums[dev::N_SHELLS + s] = s > 0 ? sums[dev::N_SHELLS + s - 1] + o[3] : o[3];
-            sums[2 * dev::N_SHELLS] = s > 0 ? std::max(sums[2 * dev::N_SHELLS], o[0]) : o[0];
         }
+        dev::fill_shell_sums(img.data() + m.off_shells + mat * dev::N_SHELLS * dev::SHELL_FLOATS,
+            img.data() + m.off_shell_sums + mat * dev::SHELL_SUM_FLOATS);
     }
     // inverse-CDF sampling tables for the Compton and Rayleigh samplers, after the
     // part of the image that the kernels stage in shared memory

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "shells.hpp"
 #include "stream_seed.hpp"
 
 namespace dxmc_gb300::dev {
@@ -152,9 +153,6 @@ __device__ __forceinline__ Real table_quantile(const float* row, int nu, Real u,
     return m_fma(fe, q1 - q0, q0);
 }
 
-constexpr int SHELL_FLOATS = 12; // binding, nElectrons, J0, photoProb, yield, lineP[3], lineE[3], pad
-constexpr int N_SHELLS = 12;
-constexpr int SHELL_SUM_FLOATS = 28; // partial sums over the shells: electrons (J0 > 0)[12], photoProb[12], highest binding energy, pad
 
 constexpr float KEV_TO_ANGSTROM = 12.398520f;
 constexpr float ELECTRON_REST_MASS = 510.9989461f;

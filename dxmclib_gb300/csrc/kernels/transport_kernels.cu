@@ -117,46 +117,6 @@ namespace {
     // cosine of the scattering angle); the direction changes in one place for all of
     // them, by an azimuth drawn last (peturb).
 
-    // Shell of a photoelectric or impulse-approximation Compton event: the first
-    // whose cumulated weight reaches u times the total.  The partial sums are taken
-    // in the same order for the total and for the search, so both use one list; above
-    // the highest binding energy of the material, where every shell takes part, the list
-    // is the LUT's (summed by the host in the same order).
-    template <class Real>
-    __device__ __forceinline__ int pick_shell(const Real (&cum)[N_SHELLS], Real u)
-    {
-        const Real sample = cum[N_SHELLS - 1] * u;
-        int idx = 0;
-#pragma unroll
-        for (int s = 0; s < N_SHELLS - 1; ++s)
-            idx += cum[s] < sample ? 1 : 0; // the sums do not decrease
-        return idx;
-    }
-
-    // The sums of a material's shells at this energy into cum: weights `which` (0: the
-    // electrons of shells with a Compton profile, 1: photoelectric).
-    template <int WHICH, class Real>
-    __device__ __forceinline__ void shell_sums(const float* L, const LutMeta& m, Real E, int material, Real (&cum)[N_SHELLS])
-    {
-        const float* ready = L + m.off_shell_sums + material * SHELL_SUM_FLOATS;
-        if (E > ready[2 * N_SHELLS]) {
-#pragma unroll
-            for (int s = 0; s < N_SHELLS; ++s)
-                cum[s] = ready[WHICH * N_SHELLS + s];
-            return;
-        }
-        const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
-        Real total = Real(0.0);
-        for (int s = 0; s < N_SHELLS; ++s) {
-            const float* sh = shells + s * SHELL_FLOATS;
-            const Real weight = WHICH == 0 ? (sh[2] > 0.0f ? Real(sh[1]) : Real(0.0)) : Real(sh[3]);
-            total += sh[0] < E ? weight : Real(0.0);
-#pragma unroll
-            for (int k = 0; k < N_SHELLS; ++k) // cum stays in registers
-                cum[k] = k == s ? total : cum[k];
-        }
-    }
-
     // ---- photoelectric (transport.hpp:216-263) ---------------------------------
     // Returns the energy imparted; `turn`: a characteristic photon of `energy` leaves
     // at angle cosA, otherwise energy is 0.
@@ -171,7 +131,7 @@ namespace {
         } else {
             const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
             Real cum[N_SHELLS] = {};
-            shell_sums<1>(L, m, E, material, cum);
+            shell_sums<1>(shells, L + m.off_shell_sums + material * SHELL_SUM_FLOATS, E, cum);
             const float* sh = shells + pick_shell(cum, up<Real>(rng.uniform())) * SHELL_FLOATS;
             const Real binding = sh[0];
             if (binding > E || binding < Real(ENERGY_CUTOFF_D))
@@ -245,7 +205,7 @@ namespace {
     {
         const float* shells = L + m.off_shells + material * N_SHELLS * SHELL_FLOATS;
         Real cum[N_SHELLS] = {};
-        shell_sums<0>(L, m, energy, material, cum);
+        shell_sums<0>(shells, L + m.off_shell_sums + material * SHELL_SUM_FLOATS, energy, cum);
         const int shell = pick_shell(cum, up<Real>(rng.uniform()));
         if (!(cum[N_SHELLS - 1] > Real(0.0)))
             return -1;

@@ -11,7 +11,7 @@ REPO = Path(__file__).resolve().parents[1]
 
 def _run(name, tmp_path):
     exe = tmp_path / name
-    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", f"-I{REPO / 'dxmclib_gb300' / 'csrc'}", f"-I{REPO / 'tests' / 'emulation'}",
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wno-unknown-pragmas", f"-I{REPO / 'dxmclib_gb300' / 'csrc'}", f"-I{REPO / 'tests' / 'emulation'}",
                         str(REPO / "tests" / "emulation" / f"{name}.cpp"), "-o", str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
@@ -20,3 +20,9 @@ def _run(name, tmp_path):
 
 def test_work_units_are_taken_whatever_the_order_of_the_lanes(tmp_path):
     _run("work_split_check", tmp_path)
+
+
+def test_shell_sums_are_in_the_precision_of_the_kernel(tmp_path):
+    """Kernels in double sum the shells' weights in double, below and above the
+    material's highest binding energy; kernels in single precision take the LUT's sums."""
+    _run("shells_check", tmp_path)
