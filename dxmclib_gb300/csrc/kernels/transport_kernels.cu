@@ -756,6 +756,7 @@ namespace {
         __device__ __forceinline__ void sync() const { __syncwarp(); }
         __device__ __forceinline__ uint64_t broadcast(uint64_t v) const { return __shfl_sync(FULL_MASK, v, 0); }
         __device__ __forceinline__ uint64_t fetch_add(unsigned long long* head) const { return atomicAdd(head, 1ull); }
+        __device__ __forceinline__ void stop(unsigned long long* head) const { atomicOr(head, static_cast<unsigned long long>(QUEUE_STOPPED)); }
     };
 
     // Photons sampled ahead for one warp (shared memory, one row per field).  All 32
@@ -1213,6 +1214,10 @@ namespace {
     __global__ void __launch_bounds__(transport_block(FAST, FORCED, PALETTE, MODEL), sizeof(Real) == 4 ? DXMC_MIN_BLOCKS_PER_SM : 2) transport_kernel(const __grid_constant__ TransportParams p)
     {
         extern __shared__ float4 smem_f4[];
+        // a job cancelled before its kernel ran takes no history (the read over the link
+        // overlaps the staging below)
+        __shared__ int cancelled;
+        const int flag = threadIdx.x == 0 && p.cancel ? *p.cancel : 0;
         // in the fast kernels a shared-memory address to the compiler (32-bit loads)
         const float* L = FAST ? reinterpret_cast<const float*>(smem_f4) : p.lut;
         size_t smem_off = 0;
@@ -1237,6 +1242,8 @@ namespace {
         float* table = nullptr; // this lane's column of the attenuation table
         if constexpr (FAST)
             table = reinterpret_cast<float*>(smem_f4 + smem_off) + threadIdx.x;
+        if (threadIdx.x == 0)
+            cancelled = flag;
         __syncthreads();
         const int lane = threadIdx.x & 31;
         const unsigned lanemask_lt = (1u << lane) - 1u;
@@ -1254,6 +1261,10 @@ namespace {
             ws = WarpState {};
             const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
             ws.next = work_unit(p.work, unit, ws.end);
+            if (cancelled) {
+                ws.next = source_total;
+                ws.end = ~0ull; // and no further unit
+            }
             ws.burst = p.woodcock_burst > 0 ? p.woodcock_burst : (sizeof(Real) == 8 ? SHORT_BURST : START_BURST);
         }
         __syncwarp();

@@ -27,11 +27,19 @@ DXMC_HD inline std::uint64_t work_unit(const WorkSplit& w, std::uint64_t unit, s
     return first;
 }
 
+// In the queue's counter: the job was cancelled, its units go to nobody any more.  The
+// count below it stays what it is.
+constexpr std::uint64_t QUEUE_STOPPED = 1ull << 63;
+// Units between two looks at the host's cancel flag, which costs a read over the link (a
+// microsecond); the warp that finds it set stops the queue for all.  A block looks once
+// before its first units, so a job cancelled while it waits does no work.
+constexpr std::uint64_t CANCEL_CHECK_UNITS = 32;
+
 // The first of the ids that a warp samples next: the rest of its unit, or a new unit,
-// the queue's next one after the first `warps`.  `ids` (next, end) is the warp's shared
-// state.  Called by all lanes of the warp, which get the same value; the caller advances
-// ids.next.  Warp: leader(), sync(), broadcast(value of the leader), fetch_add(address).
-// `cancelled` is asked by the leader for units that start as large ones.
+// the queue's next one after the first `warps`; `total` or more once there is none.
+// `ids` (next, end) is the warp's shared state.  Called by all lanes of the warp, which get
+// the same value; the caller advances ids.next.  Warp: leader(), sync(), broadcast(value of
+// the leader), fetch_add(address), stop(address).
 template <class Warp, class Ids, class Cancelled>
 DXMC_HD inline std::uint64_t next_ids(Warp& warp, Ids& ids, const WorkSplit& work, std::uint64_t warps, unsigned long long* head,
     std::uint64_t total, Cancelled&& cancelled)
@@ -41,13 +49,17 @@ DXMC_HD inline std::uint64_t next_ids(Warp& warp, Ids& ids, const WorkSplit& wor
         // every lane has read ids.end before the leader writes it
         warp.sync();
         if (warp.leader()) {
-            const std::uint64_t unit = warps + warp.fetch_add(head);
+            const std::uint64_t fetched = warp.fetch_add(head);
+            const std::uint64_t unit = warps + fetched;
             std::uint64_t end;
             next = work_unit(work, unit, end);
             ids.end = end;
-            // the host's flag costs a read over the link: not at every small unit
-            if (unit < work.large_units && cancelled())
+            if (fetched & QUEUE_STOPPED) {
                 next = total;
+            } else if (unit % CANCEL_CHECK_UNITS == 0 && cancelled()) {
+                warp.stop(head);
+                next = total;
+            }
         }
         next = warp.broadcast(next);
     }

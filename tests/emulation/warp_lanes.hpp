@@ -66,6 +66,7 @@ public:
         return value_;
     }
     std::uint64_t fetch_add(unsigned long long* head) { return (*head)++; }
+    void stop(unsigned long long* head) { *head |= 1ull << 63; }
 
 private:
     struct Lane {

@@ -48,10 +48,48 @@ void all_ids_once(const WorkSplit& work, std::uint64_t total, bool ascending)
     check(std::all_of(taken.begin(), taken.end(), [](int n) { return n == 1; }), "every id is taken once");
 }
 
+// The flag is set once `set_after` ids have been handed out; what the queue gives after that,
+// to this warp and to another one that never looks at the flag itself.
+void stops_when_cancelled(const WorkSplit& work, std::uint64_t total, std::uint64_t set_after)
+{
+    Ids ids;
+    ids.next = work_unit(work, 0, ids.end);
+    unsigned long long head = 0;
+    std::uint64_t taken = 0;
+    emulation::Warp warp;
+    warp.run(
+        [&](emulation::Warp& w, int) {
+            while (true) {
+                const std::uint64_t next = next_ids(w, ids, work, 1, &head, total, [&] { return taken >= set_after; });
+                if (next >= total)
+                    break;
+                w.sync();
+                if (w.leader()) {
+                    ids.next = next + 32;
+                    taken += 32;
+                }
+                w.sync();
+            }
+        },
+        true);
+    check(taken < set_after + CANCEL_CHECK_UNITS * std::max(work.large, work.small) + 32, "the flag is seen within a few units");
+    Ids other;
+    bool stopped = false;
+    warp.run([&](emulation::Warp& w, int) { stopped = next_ids(w, other, work, 1, &head, total, [] { return false; }) >= total; }, true);
+    check(stopped, "the queue is stopped for the other warps");
+}
+
 } // namespace
 
 int main()
 {
+    WorkSplit split;
+    stops_when_cancelled(split, 1u << 20, 0); // small units only
+    stops_when_cancelled(split, 1u << 20, 5000);
+    split.large_units = 1; // as in jobs of a few rounds: the queue hands out small ones only
+    stops_when_cancelled(split, 1u << 20, 5000);
+    split.large_units = 200; // cancelled among the last, small units
+    stops_when_cancelled(split, 1u << 20, 200 * 256 + 1000);
     for (const bool ascending : { true, false })
         for (const std::uint64_t total : { 1u, 31u, 32u, 33u, 700u, 1500u }) {
             WorkSplit work; // small units only
