@@ -324,6 +324,10 @@ struct dxmc_job {
     int* cancel_dev = nullptr;
     cudaEvent_t begin = nullptr, start = nullptr, stop = nullptr; // job begin, kernel start, kernel end
     uint64_t histories = 0;
+    // how the warps of a single-job kernel share the histories (for the progress);
+    // 0 warps: the job's counters hold histories (persistent batch, photon queue)
+    WorkSplit work;
+    uint64_t work_warps = 0;
     int tally_mode = 0;
     uint32_t tally_copies = 1; // of the records, while the job runs
     uint64_t bytes = 0;
@@ -2054,6 +2058,8 @@ cudaError_t enqueue_job(dxmc_job* j, dev::TransportParams p, int model, uint64_t
 {
     cudaError_t e = cudaSuccess;
     if (chunk == 0) {
+        j->work = p.work;
+        j->work_warps = static_cast<uint64_t>(L.grid) * (L.block / 32);
         e = record(j->start, s, capturing);
         if (e == cudaSuccess)
             e = dev::launch_transport(p, model, L.grid, L.block, L.smem, s);
@@ -3039,7 +3045,9 @@ int dxmc_gpu_job_progress(dxmc_job* j, uint64_t* started, uint64_t* total)
         cudaMemcpyDeviceToHost, ctx->result_stream));
     DXMC_CUDA(ctx, cudaStreamSynchronize(ctx->result_stream));
     const bool done = cudaEventQuery(j->stop) == cudaSuccess;
-    *started = done ? j->histories : std::min<uint64_t>(std::max(hc->next_history, hc->histories_done), j->histories);
+    // the single-job kernels' counter holds units of work beside the warps' first ones
+    const uint64_t taken = j->work_warps ? ids_taken(j->work, j->work_warps, hc->next_history & ~QUEUE_STOPPED, j->histories) : hc->next_history;
+    *started = done ? j->histories : std::min<uint64_t>(std::max<uint64_t>(taken, hc->histories_done), j->histories);
     if (total)
         *total = j->histories;
     return DXMC_OK;

@@ -27,6 +27,15 @@ DXMC_HD inline std::uint64_t work_unit(const WorkSplit& w, std::uint64_t unit, s
     return first;
 }
 
+// The ids handed out once the queue has given `fetched` units beside the first ones of
+// `warps` warps.
+inline std::uint64_t ids_taken(const WorkSplit& w, std::uint64_t warps, std::uint64_t fetched, std::uint64_t total)
+{
+    std::uint64_t end;
+    const std::uint64_t first = work_unit(w, warps + fetched, end);
+    return first < total ? first : total;
+}
+
 // In the queue's counter: the job was cancelled, its units go to nobody any more.  The
 // count below it stays what it is.
 constexpr std::uint64_t QUEUE_STOPPED = 1ull << 63;

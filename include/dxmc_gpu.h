@@ -360,7 +360,8 @@ int dxmc_gpu_job_cancel(dxmc_job* job);
 int dxmc_gpu_job_result(dxmc_job* job, int output_mode, double calibration,
     double* dose, double* variance, uint32_t* n_events, dxmc_job_stats* stats);
 /* Live progress of a running job (ProgressBar, progressbar.hpp:42-80): the
- * histories its kernels have taken so far (photons generated in the kernel) or
+ * histories its kernels have taken so far (photons generated in the kernel; the
+ * warps take their first ones, up to three quarters of a small job, at its start) or
  * queued (pre-generated photons); reads a device counter, does not wait. */
 int dxmc_gpu_job_progress(dxmc_job* job, uint64_t* histories_started, uint64_t* histories_total);
 /* Dose preview while the job runs (ProgressBar::setDoseData, progressbar.hpp:94-101):

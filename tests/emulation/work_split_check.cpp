@@ -3,6 +3,7 @@
 #include "warp_lanes.hpp"
 
 #include <algorithm>
+#include <initializer_list>
 
 using namespace dxmc_gb300;
 
@@ -19,6 +20,23 @@ void check(bool ok, const char* what)
         std::printf("FAIL %s\n", what);
         ++failures;
     }
+}
+
+// What the progress says after each unit that the queue gives: the ids handed out, up to the
+// job's total.
+void progress_counts_ids(const WorkSplit& work, std::uint64_t warps, std::uint64_t total)
+{
+    std::uint64_t end, handed = 0;
+    bool same = true;
+    for (std::uint64_t unit = 0;; ++unit) {
+        if (unit >= warps)
+            same = same && ids_taken(work, warps, unit - warps, total) == std::min(handed, total);
+        const std::uint64_t first = work_unit(work, unit, end);
+        handed += end - first;
+        if (unit > warps && first >= total)
+            break;
+    }
+    check(same, "the progress is the number of ids handed out");
 }
 
 // One warp takes all units of a job of `total` ids: every id once, all lanes the same.
@@ -83,6 +101,17 @@ void stops_when_cancelled(const WorkSplit& work, std::uint64_t total, std::uint6
 
 int main()
 {
+    for (const std::uint64_t warps : { 1u, 7u, 64u })
+        for (const std::uint64_t total : { 1u, 100u, 5000u, 100000u }) {
+            WorkSplit work;
+            progress_counts_ids(work, warps, total);
+            work.large = 96;
+            work.large_units = std::min<std::uint64_t>(warps, total / work.large);
+            progress_counts_ids(work, warps, total);
+            work.large_units = total / work.large / 2;
+            work.small = 64;
+            progress_counts_ids(work, warps, total);
+        }
     WorkSplit split;
     stops_when_cancelled(split, 1u << 20, 0); // small units only
     stops_when_cancelled(split, 1u << 20, 5000);

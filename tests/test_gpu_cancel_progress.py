@@ -1,6 +1,6 @@
-"""GPU tests of cancelling small jobs: a job cancelled while it waits behind another one
-takes no history, whichever kernel it would have run, and a job of a few rounds per warp
-stops while it runs."""
+"""GPU tests of cancelling small jobs and of their progress: a job cancelled while it waits
+behind another one takes no history, whichever kernel it would have run, a job of a few
+rounds per warp stops while it runs, and its progress is in histories."""
 from __future__ import annotations
 
 import numpy as np
@@ -65,4 +65,24 @@ def test_job_of_a_few_rounds_stops_while_it_runs(gpu_ctx, body):
     _, _, _, stats = job.result(A.OUTPUT_EV_PER_HISTORY, check=False)
     assert stats["status"] == A.DXMC_ERR_CANCELLED
     assert 0 < stats["histories"] < total
+    job.close()
+
+
+def test_progress_of_a_job_of_a_few_rounds(gpu_ctx, body):
+    """The warps take their first units, about three quarters of such a job, when its kernel
+    starts; then the progress grows with the small units that are taken."""
+    from dxmclib_gb300 import _capi as A
+    job, total = _slow_job(gpu_ctx, body)
+    seen = []
+    while True:
+        started, of = job.progress()
+        if job.wait(0) != A.DXMC_ERR_TIMEOUT:
+            break
+        assert of == total
+        if started:
+            seen.append(started)
+    assert len(seen) > 2, "the job was too short for this test"
+    assert seen == sorted(seen) and seen[-1] <= total
+    assert total // 2 < seen[0] < total
+    assert job.progress() == (total, total)
     job.close()
