@@ -66,14 +66,16 @@ constexpr int SAMPLING_LEVELS = 512;
 
 struct BatchEngines;
 
-// Page-locked, mapped host blocks that hold a job's cancel flag (byte 0) and the
-// host copy of its counters (byte 16).  Freeing page-locked memory waits for all
+// Page-locked, mapped host blocks that hold a job's cancel flag (byte 0), the
+// host copy of its counters (byte 16), written by the results, and after that the two
+// counters that a look at the progress reads (on another stream than asynchronous results).  Freeing page-locked memory waits for all
 // work on the device, which would make freeing one job wait for the jobs queued
 // after it: the blocks go back to this list and are released with the context.
 struct PinnedSlots {
     static constexpr size_t SLOT = 128;
     static constexpr int PER_CHUNK = 64;
-    static_assert(16 + sizeof(dev::JobCounters) <= SLOT, "a slot holds the flag and the counters");
+    static constexpr size_t PROGRESS_AT = 16 + sizeof(dev::JobCounters);
+    static_assert(PROGRESS_AT + 2 * sizeof(unsigned long long) <= SLOT, "a slot holds the flag, the counters and the progress");
     std::vector<void*> chunks;
     std::vector<std::pair<int*, int*>> free_slots; // (host, device) addresses
     cudaError_t take(int** host, int** device)
@@ -3039,15 +3041,17 @@ int dxmc_gpu_job_progress(dxmc_job* j, uint64_t* started, uint64_t* total)
         *started = 0;
         return DXMC_OK;
     }
-    auto* hc = reinterpret_cast<dev::JobCounters*>(reinterpret_cast<unsigned char*>(j->cancel_host) + 16);
-    // a racy snapshot of a counter the kernels only increase
-    DXMC_CUDA(ctx, cudaMemcpyAsync(&hc->next_history, &j->counters->next_history, 3 * sizeof(unsigned long long),
+    auto* seen = reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(j->cancel_host) + PinnedSlots::PROGRESS_AT);
+    static_assert(offsetof(dev::JobCounters, next_history) == 0 && offsetof(dev::JobCounters, histories_done) == 8, "copied together");
+    // a racy snapshot of counters the kernels only increase
+    DXMC_CUDA(ctx, cudaMemcpyAsync(seen, &j->counters->next_history, 2 * sizeof(unsigned long long),
         cudaMemcpyDeviceToHost, ctx->result_stream));
     DXMC_CUDA(ctx, cudaStreamSynchronize(ctx->result_stream));
+    const uint64_t next_history = seen[0], histories_done = seen[1];
     const bool done = cudaEventQuery(j->stop) == cudaSuccess;
     // the single-job kernels' counter holds units of work beside the warps' first ones
-    const uint64_t taken = j->work_warps ? ids_taken(j->work, j->work_warps, hc->next_history & ~QUEUE_STOPPED, j->histories) : hc->next_history;
-    *started = done ? j->histories : std::min<uint64_t>(std::max<uint64_t>(taken, hc->histories_done), j->histories);
+    const uint64_t taken = j->work_warps ? ids_taken(j->work, j->work_warps, next_history & ~QUEUE_STOPPED, j->histories) : next_history;
+    *started = done ? j->histories : std::min<uint64_t>(std::max(taken, histories_done), j->histories);
     if (total)
         *total = j->histories;
     return DXMC_OK;
