@@ -222,6 +222,7 @@ struct dxmc_gpu_ctx {
     PinnedSlots pinned;      // the jobs' cancel flags and counter copies
     PinnedStaging staging;   // the jobs' tables on their way to the device
     JobBufferCache job_buffers; // idle tally and queue buffers of finished jobs
+    std::vector<dxmc_job*> with_copies; // jobs that hold copies of their tally (see fits)
     // Page-locked, mapped area for the small read-backs a call waits for (palette
     // size and table, a grid's level histogram, per-material maxima).  A kernel
     // writes them there: a copy would queue on the copy engine behind an earlier
@@ -331,7 +332,9 @@ struct dxmc_job {
     WorkSplit work;
     uint64_t work_warps = 0;
     int tally_mode = 0;
-    uint32_t tally_copies = 1; // of the records, while the job runs
+    uint32_t tally_copies = 1; // of the records, while the job runs ...
+    dev::TallyRecord* more_records = nullptr; // ... all but the first of them, and their size (part of `bytes`)
+    uint64_t more_bytes = 0;
     uint64_t bytes = 0;
     bool cancelled = false;
     bool overflowed = false;
@@ -781,6 +784,7 @@ void wait_unused(dxmc_gpu_ctx* ctx, const Usage& u);
 void release_engines(dxmc_gpu_ctx* ctx);
 int wait_event(dxmc_gpu_ctx* ctx, cudaEvent_t ev, int64_t timeout_ms, const char* what);
 int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool build, const dev::MajorantGrid** out);
+bool fits(dxmc_gpu_ctx* ctx, uint64_t bytes, bool may_wait = true);
 } // namespace
 
 int dxmc_gpu_device_count(void)
@@ -960,7 +964,7 @@ try {
             return fail(ctx, DXMC_ERR_INVALID, "invalid world: direction cosines are not orthogonal");
     }
     const uint64_t bytes = n * sizeof(dev::Voxel);
-    if (ctx->in_use + bytes > ctx->budget)
+    if (!fits(ctx, bytes))
         return fail(ctx, DXMC_ERR_OOM, "world exceeds the device memory budget");
     cudaSetDevice(ctx->device);
     auto* w = new (std::nothrow) dxmc_world;
@@ -1387,6 +1391,9 @@ void free_job_device(dxmc_job* j, bool idle)
         cudaFreeAsync(j->counters, s);
     if (j->tables)
         cudaFreeAsync(j->tables, s);
+    give(j->more_records, j->more_bytes);
+    auto& with_copies = j->ctx->with_copies;
+    with_copies.erase(std::remove(with_copies.begin(), with_copies.end(), j), with_copies.end());
     if (j->staging) {
         if (!idle)
             cudaStreamSynchronize(s); // the tables copy may still be queued
@@ -1395,10 +1402,36 @@ void free_job_device(dxmc_job* j, bool idle)
     }
     j->queue = nullptr;
     j->records = nullptr;
+    j->more_records = nullptr;
     j->tally_f32 = nullptr;
     j->n_events = nullptr;
     j->counters = nullptr;
     j->tables = nullptr;
+}
+
+// Whether `bytes` more fit the context's budget.  Where they do not, the copies of pencil
+// jobs' tallies give way, which only make those jobs faster: those of jobs that have ended
+// (their copies have been added to the first) or, as members of a batch, have not been
+// launched yet, and then (may_wait) those of running jobs, once they end.
+bool fits(dxmc_gpu_ctx* ctx, uint64_t bytes, bool may_wait)
+{
+    if (!ctx->with_copies.empty())
+        cudaSetDevice(ctx->device);
+    for (int pass = 0; pass < (may_wait ? 2 : 1); ++pass)
+        for (size_t i = ctx->with_copies.size(); i-- > 0 && ctx->in_use + bytes > ctx->budget;) {
+            dxmc_job* j = ctx->with_copies[i];
+            // a stop event that was never recorded counts as complete
+            if ((pass == 0 ? cudaEventQuery(j->stop) : cudaEventSynchronize(j->stop)) != cudaSuccess)
+                continue;
+            cudaFreeAsync(j->more_records, ctx->stream);
+            ctx->in_use -= j->more_bytes;
+            j->bytes -= j->more_bytes;
+            j->more_bytes = 0;
+            j->more_records = nullptr;
+            j->tally_copies = 1;
+            ctx->with_copies.erase(ctx->with_copies.begin() + static_cast<std::ptrdiff_t>(i));
+        }
+    return ctx->in_use + bytes <= ctx->budget;
 }
 
 } // namespace
@@ -1518,7 +1551,7 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
         }
     }
     const uint64_t cell_bytes = ncell * b.bands * sizeof(float2);
-    if (ctx->in_use + cell_bytes > ctx->budget)
+    if (!fits(ctx, cell_bytes))
         return fail(ctx, DXMC_ERR_OOM, "local-majorant grid exceeds the device memory budget");
     // least recently used first, never a grid the current submission reads
     // (the cache may then hold more grids until a later submission)
@@ -1635,7 +1668,9 @@ int world_majorant(dxmc_gpu_ctx* ctx, dxmc_world* w, const dxmc_lut* lut, bool b
     // whose two scratch grids stay within MAJORANT_SCRATCH_BYTES and what the
     // context's budget leaves beside the grid and the build's other buffers (one
     // pair at a time if it leaves less)
-    const uint64_t held = ctx->in_use + cell_bytes + ncell * b.bands * (2 + sizeof(float));
+    const uint64_t build_bytes = cell_bytes + ncell * b.bands * (2 + sizeof(float));
+    fits(ctx, build_bytes + MAJORANT_SCRATCH_BYTES, false); // idle tally copies give way
+    const uint64_t held = ctx->in_use + build_bytes;
     const uint64_t room = std::min<uint64_t>(MAJORANT_SCRATCH_BYTES, ctx->budget > held ? ctx->budget - held : 0);
     const size_t group = std::clamp<size_t>(room / (2 * ncell * sizeof(float)), 1,
         std::min<size_t>(std::max<size_t>(pairs.size(), 1), dev::MAJORANT_MAX_PAIRS));
@@ -1716,7 +1751,8 @@ enum class QueueMode { own, none, shared };
 // in the 64^3 water cube took 0.20 to 0.27 ms (by where the records lay in L2), 1e8 histories 20 ms.
 // With four, blocks that take turns spread the line enough.  The copies cost a clear
 // and a pass of their own, about 0.04 ns a voxel: worth it from about one history per voxel,
-// for jobs that are not a matter of launches anyway.
+// for jobs that are not a matter of launches anyway.  They take memory that nothing else
+// needs (see fits): the choice here is a wish.
 uint32_t tally_copies(const dxmc_job_desc* jd, uint64_t histories, uint64_t voxels)
 {
     constexpr uint32_t COPIES = 4;
@@ -1847,8 +1883,9 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
     std::memcpy(tables.data() + off_btw, bt_w.data(), bt_w.size() * 4);
 
     const uint64_t nv = world->params.n_voxels;
-    const uint32_t copies = tally_mode == 1 || qmode == QueueMode::none ? 1 : tally_copies(jd, total, nv);
-    const uint64_t tally_bytes = tally_mode == 1 ? nv * 2 * sizeof(float) : copies * nv * sizeof(dev::TallyRecord);
+    uint32_t copies = tally_mode == 1 || qmode == QueueMode::none ? 1 : tally_copies(jd, total, nv);
+    const uint64_t more_bytes = (copies - 1) * nv * sizeof(dev::TallyRecord);
+    const uint64_t tally_bytes = tally_mode == 1 ? nv * 2 * sizeof(float) : nv * sizeof(dev::TallyRecord);
     const uint64_t count_bytes = tally_mode == 1 ? nv * sizeof(uint32_t) : 0; // records hold their counts
     // photon queue: chunks of 2^k histories, 48 bytes per queued photon
     const int log2_option = jd->queue_log2_chunk != 0 ? jd->queue_log2_chunk : ctx->options.queue_log2_chunk;
@@ -1861,9 +1898,9 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
         chunk = std::min<uint64_t>({ total, shared_capacity, 1ull << std::min(log2_chunk, 34) });
     const uint64_t queue_bytes = qmode == QueueMode::own ? chunk * 48 : 0;
     const uint64_t job_bytes = tally_bytes + count_bytes + table_bytes + sizeof(dev::JobCounters) + queue_bytes;
-    if (ctx->in_use + ctx->job_buffers.held + job_bytes > ctx->budget)
+    if (ctx->in_use + ctx->job_buffers.held + job_bytes + more_bytes > ctx->budget)
         ctx->job_buffers.release(ctx->stream); // idle buffers give way to the job
-    if (ctx->in_use + job_bytes > ctx->budget)
+    if (!fits(ctx, job_bytes))
         return fail(ctx, DXMC_ERR_OOM, "job exceeds the device memory budget");
 
     cudaSetDevice(ctx->device);
@@ -1872,9 +1909,12 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
         const int rc = world_majorant(ctx, world, lut, true, &grid);
         if (rc != DXMC_OK)
             return rc;
-        if (ctx->in_use + job_bytes > ctx->budget)
+        if (!fits(ctx, job_bytes))
             return fail(ctx, DXMC_ERR_OOM, "job exceeds the device memory budget");
     }
+    if (ctx->in_use + job_bytes + more_bytes > ctx->budget)
+        copies = 1; // slower, and the same results
+    ctx->with_copies.reserve(ctx->with_copies.size() + 1);
     auto* j = new (std::nothrow) dxmc_job;
     if (!j)
         return DXMC_ERR_OOM;
@@ -1882,7 +1922,6 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
     j->world = world;
     j->histories = total;
     j->tally_mode = tally_mode;
-    j->tally_copies = copies;
     j->bytes = job_bytes;
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaSuccess;
@@ -1895,6 +1934,16 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
             e = job_alloc(ctx, &j->n_events, count_bytes, s);
     } else {
         e = job_alloc(ctx, &j->records, tally_bytes, s);
+    }
+    if (e == cudaSuccess && copies > 1) {
+        if (job_alloc(ctx, &j->more_records, more_bytes, s) == cudaSuccess) {
+            j->tally_copies = copies;
+            j->more_bytes = more_bytes;
+            j->bytes += more_bytes;
+        } else { // the device has less free memory than the budget says
+            cudaGetLastError();
+            j->more_records = nullptr;
+        }
     }
     if (e == cudaSuccess)
         e = pool_alloc(ctx, &j->counters, sizeof(dev::JobCounters), s);
@@ -1910,6 +1959,8 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
         e = ctx->pinned.take(&j->cancel_host, &j->cancel_dev);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(j->records ? static_cast<void*>(j->records) : static_cast<void*>(j->tally_f32), 0, tally_bytes, s);
+    if (e == cudaSuccess && j->more_records)
+        e = cudaMemsetAsync(j->more_records, 0, more_bytes, s);
     if (e == cudaSuccess && j->n_events)
         e = cudaMemsetAsync(j->n_events, 0, count_bytes, s);
     if (e == cudaSuccess)
@@ -1959,7 +2010,8 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
     p.lut = lut->image;
     p.lut_meta = lut->meta;
     p.records = j->records;
-    p.tally_copies = copies;
+    p.more_records = j->more_records;
+    p.tally_copies = j->tally_copies;
     p.tally = nullptr;
     p.tally_f32 = j->tally_f32;
     p.n_events = j->n_events;
@@ -1997,8 +2049,8 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
     if (grid)
         p.majorant = *grid;
     p.normalize_direction = jd->direction == DXMC_DIRECTION_NORMALIZED ? 1 : 0;
-
-
+    if (j->more_records)
+        ctx->with_copies.push_back(j);
     chunk_out = chunk;
     *out = j;
     return DXMC_OK;
@@ -2084,7 +2136,7 @@ cudaError_t enqueue_job(dxmc_job* j, dev::TransportParams p, int model, uint64_t
         }
     }
     if (e == cudaSuccess && j->tally_copies > 1)
-        e = dev::launch_fold_tallies(j->records, j->world->params.n_voxels, j->tally_copies, s);
+        e = dev::launch_fold_tallies(j->records, j->more_records, j->world->params.n_voxels, j->tally_copies, s);
     if (e == cudaSuccess)
         e = record(j->stop, s, capturing);
     return e;
@@ -2317,7 +2369,7 @@ int ensure_chains(dxmc_gpu_ctx* ctx, BatchEngines& en, int chains, uint64_t capa
         if (c.queue || capacity == 0)
             continue;
         const uint64_t bytes = en.queue_capacity * 48;
-        if (ctx->in_use + bytes > ctx->budget)
+        if (!fits(ctx, bytes))
             return fail(ctx, DXMC_ERR_OOM, "batch photon queues exceed the device memory budget");
         const cudaError_t e = cudaMalloc(&c.queue, bytes);
         if (e != cudaSuccess)
@@ -2516,8 +2568,12 @@ try {
             lists[c].push_back(i);
         }
         std::vector<LaunchPlan> plans(n);
-        for (int i = 0; i < n; ++i) // occupancy queries and attributes stay outside the capture
+        for (int i = 0; i < n; ++i) {
+            // a job's tally copies may have given way to a later one
+            params[i].tally_copies = b->jobs[i]->tally_copies;
+            params[i].more_records = b->jobs[i]->more_records;
             plans[i] = plan_launch(ctx, entries[i].lut, entries[i].job, chunks[i] > 0, params[i]);
+        }
         for (int c = 0; c < chains && e == cudaSuccess; ++c) {
             if (lists[c].empty())
                 continue;
@@ -2894,7 +2950,7 @@ cudaError_t energy_of_records(dxmc_job* j, uint32_t copies, double* energy)
             j->ctx, true, (nv + PIECE - 1) / PIECE, PIECE * sizeof(dev::TallyRecord), &j->ctx->result_stream, 1,
             [&](uint64_t k, unsigned char* h, cudaStream_t s) {
                 const uint64_t first = k * PIECE;
-                return cudaMemcpyAsync(h, j->records + c * nv + first, std::min(PIECE, nv - first) * sizeof(dev::TallyRecord), cudaMemcpyDeviceToHost, s);
+                return cudaMemcpyAsync(h, (c ? j->more_records + (c - 1) * nv : j->records) + first, std::min(PIECE, nv - first) * sizeof(dev::TallyRecord), cudaMemcpyDeviceToHost, s);
             },
             [&](uint64_t k, const unsigned char* h) {
                 const uint64_t first = k * PIECE, n = std::min(PIECE, nv - first);

@@ -115,7 +115,8 @@ struct TransportParams {
     const float* lut;   // global LUT image
     LutMeta lut_meta;
     TallyRecord* records; // FP64 tallies as one record per voxel (jobs); nullptr: the arrays below
-    uint32_t tally_copies; // copies of the records, n_voxels apart, a power of two: blocks take turns (fold_tallies adds them up)
+    TallyRecord* more_records; // copies 1 .. tally_copies - 1 of the records, n_voxels apart
+    uint32_t tally_copies; // a power of two: blocks take turns (fold_tallies adds them up)
     uint32_t pad_copies;
     double* tally;      // interleaved (energy, energy^2) per voxel, FP64 (with n_events; the no-allocation path)
     float* tally_f32;   // interleaved, FP32 tally mode
@@ -224,8 +225,8 @@ TransportVariant transport_variant(const TransportParams& p, int model, bool que
 int transport_max_blocks_per_sm(const TransportVariant& v, int block, size_t smem);
 // dynamic shared memory the transport kernel needs
 size_t transport_smem_bytes(const TransportVariant& v, const LutMeta& meta, bool lut_in_smem);
-// Adds the copies of a job's tally records to the first one.
-cudaError_t launch_fold_tallies(TallyRecord* records, uint64_t n, uint32_t copies, cudaStream_t stream);
+// Adds the copies 1 .. copies - 1 of a job's tally records, `more`, to the first one.
+cudaError_t launch_fold_tallies(TallyRecord* records, const TallyRecord* more, uint64_t n, uint32_t copies, cudaStream_t stream);
 // Post-processing of the tallies into dose / variance (densities from the world's layout).
 // dose, variance and counts_out may be device memory or page-locked host memory
 // (written through its device mapping); counts_out, if not null, gets a copy of counts,

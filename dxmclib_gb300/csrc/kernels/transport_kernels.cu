@@ -49,7 +49,8 @@ namespace {
     // The copy of the records that this block adds to.
     __device__ __forceinline__ TallyRecord* tally_records(const TransportParams& p)
     {
-        return p.records + (blockIdx.x & (p.tally_copies - 1)) * p.world.n_voxels;
+        const uint32_t copy = blockIdx.x & (p.tally_copies - 1);
+        return copy ? p.more_records + (copy - 1) * p.world.n_voxels : p.records;
     }
 
     template <bool FAST, class Real>
@@ -1552,13 +1553,13 @@ namespace {
     }
 
     // Copies 1 .. copies - 1 of the records added to copy 0, in that order.
-    __global__ void fold_tallies_kernel(TallyRecord* __restrict__ rec, uint64_t n, uint32_t copies)
+    __global__ void fold_tallies_kernel(TallyRecord* __restrict__ rec, const TallyRecord* __restrict__ more, uint64_t n, uint32_t copies)
     {
         for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
             uint32_t events = 0;
             double e = 0.0, ee = 0.0;
             for (uint32_t c = 1; c < copies; ++c) {
-                const TallyRecord r = rec[c * n + i];
+                const TallyRecord r = more[(c - 1) * n + i];
                 events += r.events;
                 e += r.energy;
                 ee += r.energy2;
@@ -1866,11 +1867,11 @@ cudaError_t launch_postprocess(const double* tally, const WorldParams& w, uint64
     return cudaGetLastError();
 }
 
-cudaError_t launch_fold_tallies(TallyRecord* records, uint64_t n, uint32_t copies, cudaStream_t stream)
+cudaError_t launch_fold_tallies(TallyRecord* records, const TallyRecord* more, uint64_t n, uint32_t copies, cudaStream_t stream)
 {
     const int block = 256;
     const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 152ull * 8));
-    fold_tallies_kernel<<<grid, block, 0, stream>>>(records, n, copies);
+    fold_tallies_kernel<<<grid, block, 0, stream>>>(records, more, n, copies);
     return cudaGetLastError();
 }
 
