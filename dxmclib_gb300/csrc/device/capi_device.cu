@@ -6,6 +6,7 @@
 
 #include "../host/lut_builder.hpp"
 #include "../kernels/transport.cuh"
+#include "preview.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -335,6 +336,7 @@ struct dxmc_job {
     uint32_t tally_copies = 1; // of the records, while the job runs ...
     dev::TallyRecord* more_records = nullptr; // ... all but the first of them, and their size (part of `bytes`)
     uint64_t more_bytes = 0;
+    cudaEvent_t swept = nullptr; // jobs with copies: the transport kernel's end, before they are added up
     uint64_t bytes = 0;
     bool cancelled = false;
     bool overflowed = false;
@@ -1392,6 +1394,9 @@ void free_job_device(dxmc_job* j, bool idle)
     if (j->tables)
         cudaFreeAsync(j->tables, s);
     give(j->more_records, j->more_bytes);
+    if (j->swept)
+        cudaEventDestroy(j->swept);
+    j->swept = nullptr;
     auto& with_copies = j->ctx->with_copies;
     with_copies.erase(std::remove(with_copies.begin(), with_copies.end(), j), with_copies.end());
     if (j->staging) {
@@ -1940,6 +1945,7 @@ int prepare_job(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* lut, const dxmc_
             j->tally_copies = copies;
             j->more_bytes = more_bytes;
             j->bytes += more_bytes;
+            e = cudaEventCreateWithFlags(&j->swept, cudaEventDisableTiming);
         } else { // the device has less free memory than the budget says
             cudaGetLastError();
             j->more_records = nullptr;
@@ -2135,6 +2141,8 @@ cudaError_t enqueue_job(dxmc_job* j, dev::TransportParams p, int model, uint64_t
                 e = dev::launch_transport(p, model, L.grid, L.block, L.smem, s);
         }
     }
+    if (e == cudaSuccess && j->tally_copies > 1)
+        e = record(j->swept, s, capturing);
     if (e == cudaSuccess && j->tally_copies > 1)
         e = dev::launch_fold_tallies(j->records, j->more_records, j->world->params.n_voxels, j->tally_copies, s);
     if (e == cudaSuccess)
@@ -3128,15 +3136,12 @@ try {
         std::fill(energy, energy + nv, 0.0);
         return DXMC_OK;
     }
-    // the energy sum of each 32-byte tally record, over the copies of a job that still runs;
-    // if it ended meanwhile (and its copies were added to the first), that one again
-    for (bool ended = cudaEventQuery(j->stop) == cudaSuccess;;) {
-        const uint32_t copies = ended ? 1 : j->tally_copies;
-        DXMC_CUDA(ctx, energy_of_records(j, copies, energy));
-        if (copies == 1 || cudaEventQuery(j->stop) != cudaSuccess)
-            break;
-        ended = true;
-    }
+    // the energy sum of each 32-byte tally record, over the copies of a job that still runs
+    const cudaError_t e = read_tally(
+        j->tally_copies, [&] { return cudaEventQuery(j->stop) == cudaSuccess; }, [&] { return cudaEventQuery(j->swept) == cudaSuccess; },
+        [&] { return cudaEventSynchronize(j->stop); }, [&](uint32_t copies) { return energy_of_records(j, copies, energy); });
+    if (e != cudaSuccess)
+        return cuda_fail(ctx, e, "dose preview");
     return DXMC_OK;
 } catch (...) {
     return exception_status(j ? j->ctx : nullptr);

@@ -1,6 +1,7 @@
-"""CPU tests of warp-level device code with the lanes of a warp advancing one at a
-time (tests/emulation): the code is compiled for the host from the kernels' own
-headers."""
+"""CPU tests of code of the kernels and of their host side in orders of events that a GPU
+run cannot be made to take (tests/emulation): lanes of a warp that advance one at a
+time, a preview beside the kernel that adds up the tally's copies.  The code is compiled
+for the host from the library's own headers."""
 from __future__ import annotations
 
 import subprocess
@@ -26,3 +27,7 @@ def test_shell_sums_are_in_the_precision_of_the_kernel(tmp_path):
     """Kernels in double sum the shells' weights in double, below and above the
     material's highest binding energy; kernels in single precision take the LUT's sums."""
     _run("shells_check", tmp_path)
+
+
+def test_preview_counts_no_copy_twice(tmp_path):
+    _run("preview_check", tmp_path)
