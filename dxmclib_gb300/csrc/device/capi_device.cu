@@ -2834,10 +2834,12 @@ constexpr uint64_t RESULT_PIECES = 4; // 629 MB: 0.6 ms less than in one
 constexpr uint64_t DIRECT_RESULT_BYTES = 16ull << 20; // written over the link by the kernel: 0.09 ms at most
 
 // Blocks and threads of such a transfer.  `locked`: the caller holds the context's mutex.
-// enqueue(k, block, stream) queues piece k into a block, consume(k, block)
-// takes it from there; each thread has a block of its own and takes the next piece.
-cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, size_t block_bytes, const cudaStream_t* streams, int n_streams,
-    const std::function<cudaError_t(uint64_t, unsigned char*, cudaStream_t)>& enqueue,
+// enqueue(k, block) queues piece k into a block on stream s, consume(k, block)
+// takes it from there; each thread has a block of its own and takes the next piece.  The
+// result stream, on which nothing waits for a job that runs: pieces spread over the streams of
+// asynchronous results waited for those of jobs that had not ended.
+cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, size_t block_bytes, cudaStream_t s,
+    const std::function<cudaError_t(uint64_t, unsigned char*)>& enqueue,
     const std::function<void(uint64_t, const unsigned char*)>& consume)
 {
     const int cores = static_cast<int>(std::max(1u, std::thread::hardware_concurrency() / 2));
@@ -2868,9 +2870,8 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
     auto work = [&](int t) {
         Block& b = blocks[t];
         cudaSetDevice(ctx->device);
-        cudaStream_t s = streams[t % n_streams];
         for (uint64_t k; failed.load() == cudaSuccess && (k = next.fetch_add(1)) < pieces;) {
-            cudaError_t we = enqueue(k, static_cast<unsigned char*>(b.host), s);
+            cudaError_t we = enqueue(k, static_cast<unsigned char*>(b.host));
             if (we == cudaSuccess)
                 we = cudaEventRecord(b.done, s);
             if (we == cudaSuccess)
@@ -2908,25 +2909,24 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
     return e;
 }
 
-// Post-processed results in device memory, complete once `ready` has happened.
+// Post-processed results in device memory, complete in the order of the result stream.
 struct StagedResults {
     unsigned char* dose = nullptr;
     unsigned char* variance = nullptr;
     unsigned char* counts = nullptr;
-    cudaEvent_t ready = nullptr;
 };
 
 cudaError_t results_to_pageable(dxmc_job* j, const StagedResults& r, double* dose, double* variance, uint32_t* counts)
 {
+    cudaStream_t s = j->ctx->result_stream;
     const uint64_t nv = j->world->params.n_voxels;
     constexpr size_t VAR_AT = PAGEABLE_PIECE * sizeof(double), COUNT_AT = 2 * VAR_AT;
     return transfer_pieces(
-        j->ctx, false, (nv + PAGEABLE_PIECE - 1) / PAGEABLE_PIECE, COUNT_AT + PAGEABLE_PIECE * sizeof(uint32_t), j->ctx->async_streams,
-        dxmc_gpu_ctx::ASYNC_STREAMS,
-        [&](uint64_t k, unsigned char* h, cudaStream_t s) {
+        j->ctx, false, (nv + PAGEABLE_PIECE - 1) / PAGEABLE_PIECE, COUNT_AT + PAGEABLE_PIECE * sizeof(uint32_t), s,
+        [&](uint64_t k, unsigned char* h) {
             const uint64_t first = k * PAGEABLE_PIECE, n = std::min(PAGEABLE_PIECE, nv - first);
-            cudaError_t e = cudaStreamWaitEvent(s, r.ready, 0);
-            if (e == cudaSuccess && dose)
+            cudaError_t e = cudaSuccess;
+            if (dose)
                 e = cudaMemcpyAsync(h, r.dose + first * sizeof(double), n * sizeof(double), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess && variance)
                 e = cudaMemcpyAsync(h + VAR_AT, r.variance + first * sizeof(double), n * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -2950,13 +2950,14 @@ cudaError_t results_to_pageable(dxmc_job* j, const StagedResults& r, double* dos
 // voxels, and a kernel would wait for the transport's blocks), picked apart by the host.
 cudaError_t energy_of_records(dxmc_job* j, uint32_t copies, double* energy)
 {
+    cudaStream_t s = j->ctx->result_stream;
     const uint64_t nv = j->world->params.n_voxels;
     constexpr uint64_t PIECE = 32 * 1024;
     cudaError_t e = cudaSuccess;
     for (uint32_t c = 0; c < copies && e == cudaSuccess; ++c)
         e = transfer_pieces(
-            j->ctx, true, (nv + PIECE - 1) / PIECE, PIECE * sizeof(dev::TallyRecord), &j->ctx->result_stream, 1,
-            [&](uint64_t k, unsigned char* h, cudaStream_t s) {
+            j->ctx, true, (nv + PIECE - 1) / PIECE, PIECE * sizeof(dev::TallyRecord), s,
+            [&](uint64_t k, unsigned char* h) {
                 const uint64_t first = k * PIECE;
                 return cudaMemcpyAsync(h, (c ? j->more_records + (c - 1) * nv : j->records) + first, std::min(PIECE, nv - first) * sizeof(dev::TallyRecord), cudaMemcpyDeviceToHost, s);
             },
@@ -3042,7 +3043,6 @@ try {
                 cudaEventDestroy(done);
             return cuda_fail(ctx, e, "result copy");
         }
-        staged.ready = done;
     }
     cudaError_t e = cudaSuccess;
     try {
