@@ -7,6 +7,7 @@
 #include "../host/lut_builder.hpp"
 #include "../kernels/transport.cuh"
 #include "preview.hpp"
+#include "worker_team.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -18,7 +19,6 @@
 #include <new>
 #include <stdexcept>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -182,6 +182,8 @@ struct PinnedStaging {
             l.pop_back();
             return cudaSuccess;
         }
+        l.reserve(blocks.size() + 1); // giving blocks back allocates nothing
+        blocks.reserve(blocks.size() + 1);
         const cudaError_t e = cudaHostAlloc(p, *cls, cudaHostAllocDefault);
         if (e == cudaSuccess)
             blocks.push_back(*p);
@@ -2849,26 +2851,45 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
         size_t cls = 0;
         cudaEvent_t done = nullptr;
     };
-    std::vector<Block> blocks(threads);
-    std::vector<std::thread> team;
-    team.reserve(threads);
+    struct Blocks { // given back on every way out
+        dxmc_gpu_ctx* ctx;
+        bool locked;
+        std::vector<Block> list;
+        std::unique_lock<std::mutex> lock() const
+        {
+            std::unique_lock<std::mutex> l(ctx->mutex, std::defer_lock);
+            if (!locked)
+                l.lock();
+            return l;
+        }
+        ~Blocks()
+        {
+            const auto held = lock();
+            for (Block& b : list) {
+                if (b.done)
+                    cudaEventDestroy(b.done);
+                if (b.host)
+                    ctx->staging.give(b.host, b.cls);
+            }
+        }
+    } blocks { ctx, locked, std::vector<Block>(threads) };
     cudaError_t e = cudaSuccess;
     {
-        std::unique_lock<std::mutex> lock(ctx->mutex, std::defer_lock);
-        if (!locked)
-            lock.lock();
+        const auto held = blocks.lock();
         cudaSetDevice(ctx->device);
-        for (Block& b : blocks) {
+        for (Block& b : blocks.list) {
             if (e == cudaSuccess)
                 e = ctx->staging.take(block_bytes, &b.host, &b.cls);
             if (e == cudaSuccess)
                 e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
         }
     }
+    if (e != cudaSuccess)
+        return e;
     std::atomic<uint64_t> next { 0 };
-    std::atomic<int> failed { static_cast<int>(e) };
-    auto work = [&](int t) {
-        Block& b = blocks[t];
+    std::atomic<int> failed { cudaSuccess };
+    run_team(threads, [&](int t) {
+        Block& b = blocks.list[t];
         cudaSetDevice(ctx->device);
         for (uint64_t k; failed.load() == cudaSuccess && (k = next.fetch_add(1)) < pieces;) {
             cudaError_t we = enqueue(k, static_cast<unsigned char*>(b.host));
@@ -2883,30 +2904,8 @@ cudaError_t transfer_pieces(dxmc_gpu_ctx* ctx, bool locked, uint64_t pieces, siz
             }
             consume(k, static_cast<const unsigned char*>(b.host));
         }
-    };
-    if (e == cudaSuccess) {
-        for (int t = 1; t < threads; ++t) {
-            try {
-                team.emplace_back(work, t);
-            } catch (const std::system_error&) {
-                break; // no more threads: those there are take all pieces
-            }
-        }
-        work(0);
-        for (auto& t : team)
-            t.join();
-        e = static_cast<cudaError_t>(failed.load());
-    }
-    std::unique_lock<std::mutex> lock(ctx->mutex, std::defer_lock);
-    if (!locked)
-        lock.lock();
-    for (Block& b : blocks) {
-        if (b.done)
-            cudaEventDestroy(b.done);
-        if (b.host)
-            ctx->staging.give(b.host, b.cls);
-    }
-    return e;
+    });
+    return static_cast<cudaError_t>(failed.load());
 }
 
 // Post-processed results in device memory, complete in the order of the result stream.

@@ -12,7 +12,7 @@ REPO = Path(__file__).resolve().parents[1]
 
 def _run(name, tmp_path):
     exe = tmp_path / name
-    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wno-unknown-pragmas", f"-I{REPO / 'dxmclib_gb300' / 'csrc'}", f"-I{REPO / 'tests' / 'emulation'}",
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-pthread", "-Wno-unknown-pragmas", f"-I{REPO / 'dxmclib_gb300' / 'csrc'}", f"-I{REPO / 'tests' / 'emulation'}",
                         str(REPO / "tests" / "emulation" / f"{name}.cpp"), "-o", str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
@@ -31,3 +31,8 @@ def test_shell_sums_are_in_the_precision_of_the_kernel(tmp_path):
 
 def test_preview_counts_no_copy_twice(tmp_path):
     _run("preview_check", tmp_path)
+
+
+def test_team_of_threads_where_memory_runs_out(tmp_path):
+    """Fewer threads do the same work; the C ABI never ends the process for want of memory."""
+    _run("worker_team_check", tmp_path)
