@@ -188,15 +188,25 @@ struct TransportVariant {
     bool forced = true;   // forced photoelectric scoring (a measurement map)
     // The options of nearly every job: FP32 transport with the FP64 record tally (mode 0),
     // local majorants, photons sampled in the kernel, the reference's directions, and a LUT
-    // of at most ATT_TABLE_MATERIALS materials staged in shared memory.  Compiled apart,
+    // of at most ATT_TABLE_MATERIALS materials staged in shared memory beside the table (see
+    // FAST_SHARED_BYTES).  Compiled apart,
     // the kernel tests none of these in its loop and keeps a per-lane attenuation table.
     bool fast = false;
 };
-// The attenuation table of the fast kernels: one float per material and lane of a block.
-// Eight materials cover the usual segmentations (the workloads use one to four)
-// in 1 KB per warp; filling a column costs about 20 instructions per material
-// when a photon's energy changes, which beyond eight exceeds what it saves.
+// The attenuation table of the fast kernels: one float per material and lane of a block,
+// 1 KB per warp at eight materials; filling a column costs about 20 instructions per material
+// when a photon's energy changes.
 constexpr int ATT_TABLE_MATERIALS = 8;
+// Shared memory of an SM that the resident blocks of a fast kernel may take, which the
+// LUT's size decides.  With more than 196 KB the SM is left 28 KB of L1 instead of 60, and
+// the table costs more in voxel and cell reads than it saves; the impulse approximation,
+// with more arithmetic for its reads, gains up to the point where a block fewer is resident.
+// Where the general kernel does not fit either, forced scoring still gains.  With the table
+// / without, LUTs up to 150 keV: CT 512 x 512 x 100 of 2e7 histories 2.14 / 2.33 ms at five
+// materials (184 KB), 2.42 / 2.30 at six (205 KB); DX 160^3 of 5e6 with forced scoring
+// 0.89 / 0.93 at four, 1.14 / 0.94 at six, 1.05 / 1.11 at eight; with the impulse
+// approximation 0.88 / 0.94 at six (215 KB), 1.01 / 0.99 at seven (239 KB).
+constexpr size_t FAST_SHARED_BYTES = 196 * 1024, FAST_SHARED_BYTES_IA = 228 * 1024;
 constexpr int TRANSPORT_THREADS = 288; // largest block of the single-job kernels
 // Default block of a variant, four of which fill an SM's registers (two in FP64).  Where
 // 56 registers a thread are enough, nine warps a block: the 36 warps of an SM hide more of

@@ -1752,6 +1752,17 @@ TransportVariant transport_variant(const TransportParams& p, int model, bool que
     v.forced = p.world.has_measurement != 0;
     v.fast = p.precision != 1 && p.lut_meta.n_materials <= ATT_TABLE_MATERIALS && p.lut_in_smem && p.majorant.cells && p.records && p.tally_mode == 0
         && !p.normalize_direction && !queued;
+    if (v.fast) {
+        const size_t most = model == 2 ? FAST_SHARED_BYTES_IA : FAST_SHARED_BYTES;
+        const auto resident = [&](bool fast) { // shared memory of an SM's blocks
+            constexpr size_t PER_WARP = sizeof(WarpState) + sizeof(PhotonPool<float>), RESERVED = 1024;
+            TransportVariant u = v;
+            u.fast = fast;
+            const int warps = transport_block(fast, v.forced, v.palette, model) / 32;
+            return DXMC_MIN_BLOCKS_PER_SM * (transport_smem_bytes(u, p.lut_meta, true) + warps * PER_WARP + RESERVED);
+        };
+        v.fast = resident(true) <= most || (v.forced && resident(false) > most);
+    }
     return v;
 }
 
