@@ -2093,8 +2093,12 @@ LaunchPlan plan_launch(dxmc_gpu_ctx* ctx, const dxmc_lut* lut, const dxmc_job_de
     p.lut_in_smem = lut_bytes <= smem_limit ? 1 : 0;
     const dev::TransportVariant variant = dev::transport_variant(p, model, queued);
     L.smem = dev::transport_smem_bytes(variant, lut->meta, p.lut_in_smem != 0);
-    L.block = jd->block_size == 128 || jd->block_size == 256 ? jd->block_size
-                                                              : (ctx->options.block_size > 0 ? ctx->options.block_size : dev::transport_block(variant.fast, variant.forced, variant.palette, model));
+    if (jd->block_size == 128 || jd->block_size == 256)
+        L.block = jd->block_size;
+    else if (ctx->options.block_size > 0)
+        L.block = whole_warps(ctx->options.block_size);
+    else
+        L.block = dev::transport_block(variant.fast, variant.forced, variant.palette, model);
     // also sets the kernel's dynamic shared-memory limit for this launch
     const int occ = dev::transport_max_blocks_per_sm(variant, L.block, L.smem);
     int per_sm = jd->blocks_per_sm > 0 ? std::min(jd->blocks_per_sm, std::max(occ, 1))

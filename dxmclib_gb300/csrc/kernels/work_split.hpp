@@ -17,6 +17,11 @@ struct WorkSplit {
     std::uint32_t small = 32;
 };
 
+// Threads of a block for a wish of the caller's: whole warps.  A kernel whose last warp has
+// fewer lanes would give that warp the units of the next block's first, and wait for idle
+// lanes that it does not have.
+inline int whole_warps(int threads) { return threads > 32 ? (threads + 31) / 32 * 32 : 32; }
+
 // The ids of one unit of a job's work; a unit past the end starts at or after the job's
 // last id.
 DXMC_HD inline std::uint64_t work_unit(const WorkSplit& w, std::uint64_t unit, std::uint64_t& end)

@@ -243,7 +243,7 @@ typedef struct dxmc_job dxmc_job;
 
 typedef struct dxmc_gpu_options {
     int32_t device;          /* CUDA device ordinal */
-    int32_t block_size;      /* threads per block, 0 = default (256; 288 where 56 registers a thread are enough) */
+    int32_t block_size;      /* threads per block, rounded up to whole warps; 0 = default (256; 288 where 56 registers a thread are enough) */
     int32_t blocks_per_sm;   /* resident blocks per SM, 0 = occupancy-derived */
     int32_t tally_mode;      /* DXMC_TALLY_* */
     uint64_t memory_budget;  /* admission budget in bytes, 0 = 90% of free memory */

@@ -112,6 +112,10 @@ int main()
             work.small = 64;
             progress_counts_ids(work, warps, total);
         }
+    for (int threads = 1; threads <= 256; ++threads) {
+        const int block = whole_warps(threads);
+        check(block % 32 == 0 && block >= threads && block < threads + 32, "a block is whole warps");
+    }
     WorkSplit split;
     stops_when_cancelled(split, 1u << 20, 0); // small units only
     stops_when_cancelled(split, 1u << 20, 5000);
