@@ -2540,7 +2540,7 @@ try {
             c.n_items[model] = n_items - c.item_base[model];
         }
         c.chunk = (opt && opt->item_histories > 0 ? static_cast<uint64_t>(opt->item_histories) : DEFAULT_BATCH_CHUNK) / 32 * 32;
-        c.chunk = std::max<uint64_t>(32, c.chunk);
+        c.chunk = std::clamp<uint64_t>(c.chunk, 32, 65536); // the warps' counters are 32 bits wide between chunks
         const int regen = opt && opt->regen_threshold > 0 ? opt->regen_threshold
                                                           : (ctx->options.regen_threshold > 0 ? ctx->options.regen_threshold : DEFAULT_REGEN_THRESHOLD);
         const int inter = opt && opt->interact_threshold > 0 ? opt->interact_threshold

@@ -588,21 +588,41 @@ namespace {
         uint32_t steps, deposits, histories;     // since they were last added to the job's counters
         unsigned int overflows, forced_deposits; // rare events, by shared atomics
         int burst;                               // flights per iteration
+        uint64_t carried[3];                     // steps, histories and deposits beyond 32 bits
     };
+
+    // A warp's counters are 32 bits wide, a job's 64: lane 0 empties them, between units of work,
+    // once one is beyond CARRY, while the steps of a unit and of the photons in flight still
+    // fit (and the burst's rule, in 32 bits as well).
+    constexpr uint32_t CARRY = 1u << 24;
+    static_assert(CARRY + (256 + 2 * 32) * (MAX_STEPS_PER_HISTORY + 64ull) <= 0xffffffffull, "no counter of a warp wraps");
+    __device__ __forceinline__ void carry_counters(WarpState& ws)
+    {
+        if ((ws.histories | ws.steps) >= CARRY) {
+            ws.carried[0] += ws.steps;
+            ws.carried[1] += ws.histories;
+            ws.carried[2] += atomicExch(&ws.deposits, 0u); // the lanes add to it
+            ws.carried[2] += atomicExch(&ws.forced_deposits, 0u);
+            ws.steps = ws.histories = 0;
+        }
+    }
 
     // Adds the warp's counters to the job's and clears them.  Called by all 32 lanes.
     __device__ __forceinline__ void add_counters(WarpState& ws, JobCounters* c)
     {
         __syncwarp();
         if ((threadIdx.x & 31) == 0) {
-            if (ws.steps)
-                atomicAdd(&c->steps, static_cast<unsigned long long>(ws.steps));
-            if (ws.deposits + ws.forced_deposits)
-                atomicAdd(&c->deposits, static_cast<unsigned long long>(ws.deposits) + ws.forced_deposits);
+            const uint64_t steps = ws.carried[0] + ws.steps, histories = ws.carried[1] + ws.histories;
+            const uint64_t deposits = ws.carried[2] + ws.deposits + ws.forced_deposits;
+            if (steps)
+                atomicAdd(&c->steps, static_cast<unsigned long long>(steps));
+            if (deposits)
+                atomicAdd(&c->deposits, static_cast<unsigned long long>(deposits));
             if (ws.overflows)
                 atomicAdd(&c->overflows, static_cast<unsigned long long>(ws.overflows));
-            if (ws.histories)
-                atomicAdd(&c->histories_done, static_cast<unsigned long long>(ws.histories));
+            if (histories)
+                atomicAdd(&c->histories_done, static_cast<unsigned long long>(histories));
+            ws.carried[0] = ws.carried[1] = ws.carried[2] = 0;
             ws.steps = ws.deposits = ws.histories = 0;
             ws.overflows = ws.forced_deposits = 0;
         }
@@ -1281,7 +1301,7 @@ namespace {
                     const int pooled = ws.pooled;
                     if (pooled == 0) {
                         // a unit of the job is done: the job's progress, and the next unit
-                        if (ws.next >= ws.end && ws.histories >= PUBLISH_HISTORIES)
+                        if (ws.next >= ws.end && (ws.histories >= PUBLISH_HISTORIES || ws.steps >= CARRY))
                             add_counters(ws, p.counters);
                         const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
                         DeviceWarp self;
@@ -1445,8 +1465,10 @@ namespace {
                     while (need) {
                         if (next >= end) {
                             unsigned long long first = 0;
-                            if (lane == 0)
+                            if (lane == 0) {
                                 first = atomicAdd(&p.counters->next_history, static_cast<unsigned long long>(chunk));
+                                carry_counters(ws);
+                            }
                             next = __shfl_sync(FULL_MASK, first, 0);
                             end = min(next + chunk, histories);
                             if (next >= end) {
