@@ -10,7 +10,7 @@ model):
 * ``regen_threshold`` -- how many lanes of a warp must be idle before they are
   refilled together (the refill cadence);
 * ``interact_threshold`` -- how many lanes must wait for an interaction before
-  the per-type interaction passes run (the event-sorting cadence);
+  the interaction pass runs (the event-sorting cadence);
 * ``blocks_per_sm`` -- resident blocks per SM (occupancy);
 * ``block_size`` -- threads per block (128 or 256);
 * ``woodcock_burst`` -- Woodcock steps a lane may take per loop iteration before

@@ -30,7 +30,7 @@ cudaError_t preload(int device); // noalloc.cu
 }
 
 // Warp scheduling of the transport kernel: refill idle lanes once this many
-// are idle; run the per-type interaction passes once this many lanes wait.
+// are idle; run the interaction pass once this many lanes wait.
 constexpr int DEFAULT_REGEN_THRESHOLD = 8;        // photons generated in the transport kernel
 constexpr int DEFAULT_INTERACT_THRESHOLD = 8;
 constexpr int DEFAULT_QUEUE_REGEN_THRESHOLD = 4;  // photons taken from the pre-generated queue
@@ -69,9 +69,10 @@ struct BatchEngines;
 
 // Page-locked, mapped host blocks that hold a job's cancel flag (byte 0), the
 // host copy of its counters (byte 16), written by the results, and after that the two
-// counters that a look at the progress reads (on another stream than asynchronous results).  Freeing page-locked memory waits for all
-// work on the device, which would make freeing one job wait for the jobs queued
-// after it: the blocks go back to this list and are released with the context.
+// counters that a look at the progress reads (on another stream than asynchronous
+// results).  Freeing page-locked memory waits for all work on the device, which would
+// make freeing one job wait for the jobs queued after it: the blocks go back to this
+// list and are released with the context.
 struct PinnedSlots {
     static constexpr size_t SLOT = 128;
     static constexpr int PER_CHUNK = 64;
@@ -207,7 +208,7 @@ struct dxmc_gpu_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t result_stream = nullptr; // results a call waits for, progress and preview
     // asynchronous results: each job's on the next stream, so that a finished job's results
-    // do not wait for those of a job that still runs
+    // seldom wait for those of a job that still runs
     static constexpr int ASYNC_STREAMS = 4;
     cudaStream_t async_streams[ASYNC_STREAMS] {};
     cudaStream_t copy_streams[ASYNC_STREAMS] {}; // copies of large results, beside the later pieces' kernels
@@ -291,7 +292,7 @@ struct dxmc_world {
     uint64_t bytes = 0;
     dev::WorldParams params {};
     // the last use of the world by single jobs on the context stream and by the
-    // post-processing of asynchronous results on the result stream: freeing the
+    // post-processing of asynchronous results on their streams: freeing the
     // world waits for these, not for unrelated work; a world used by a batch
     // (chain or engine streams) waits for every stream of the context
     Usage usage;

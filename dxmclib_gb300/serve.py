@@ -20,7 +20,7 @@ This module adds the serving layer around the same transport:
   on the GPU as soon as memory and a chain free up (continuous batching);
 * finished jobs are collected by a collector thread in groups: each job's
   post-processing and copies into page-locked buffers from a pool are queued
-  behind it on the result stream (asynchronous results), then the group is
+  behind it (asynchronous results), then the group is
   waited for, so that results stream back over the link without a host round
   trip per job; each job's device memory is released once its copies are done,
   and the latency from arrival to result is recorded for p50 / p99.
@@ -238,7 +238,8 @@ class GpuBackend:
 
     def job_bytes(self, req: ServeRequest) -> int:
         n = int(req.world.size())
-        # one 32-byte FP64 tally record per voxel, the job's tables and counters
+        # one 32-byte FP64 tally record per voxel, the job's tables and counters (the copies of
+        # a pencil job's tally are taken only where there is room, and give way)
         return n * 32 + 80 * len(req.exposures) + (1 << 20)
 
     def result_bytes(self, n: int):

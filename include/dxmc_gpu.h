@@ -248,7 +248,7 @@ typedef struct dxmc_gpu_options {
     int32_t tally_mode;      /* DXMC_TALLY_* */
     uint64_t memory_budget;  /* admission budget in bytes, 0 = 90% of free memory */
     int32_t regen_threshold; /* refill finished lanes of a warp once this many are idle; 0 = default */
-    int32_t interact_threshold; /* run the per-type interaction passes once this many lanes wait; 0 = default */
+    int32_t interact_threshold; /* run the interaction pass once this many lanes wait; 0 = default */
     int32_t queue_log2_chunk;   /* n > 0: photons are pre-generated in chunks of 2^n histories (48 B per
                                    photon); 0 = default (generated inside the transport kernel); -1 = inside */
     int32_t tracking;           /* DXMC_TRACKING_* of jobs that leave theirs at DEFAULT */
@@ -448,7 +448,7 @@ int dxmc_gpu_transport_noalloc(dxmc_gpu_ctx* ctx, dxmc_world* world, dxmc_lut* l
 
 /* Asynchronous results.  dxmc_gpu_job_result_async queues the post-processing
  * (output_mode and calibration as dxmc_gpu_job_result) and the copies into the
- * caller's buffers on the context's result stream, ordered after the job's
+ * caller's buffers on a stream of the context, ordered after the job's
  * kernel, and returns at once: the caller may submit the next job meanwhile and
  * the copies run on the copy engine beside its transport.  result_type
  * DXMC_RESULT_F64 writes double dose / variance (Result<double>, 20 bytes per
